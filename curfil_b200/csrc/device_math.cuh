@@ -40,6 +40,16 @@ struct FeatParams {
     uint8_t type, ch1, ch2, pad;
 };
 
+// bits 0..15 of v spread to the even bit positions (Morton order)
+__device__ __forceinline__ unsigned long long spread_bits(uint32_t v) {
+    unsigned long long x = v & 0xFFFFu;
+    x = (x | (x << 8)) & 0x00FF00FFull;
+    x = (x | (x << 4)) & 0x0F0F0F0Full;
+    x = (x | (x << 2)) & 0x33333333ull;
+    x = (x | (x << 1)) & 0x55555555ull;
+    return x;
+}
+
 __device__ __forceinline__ double dnan() { return __longlong_as_double(0x7ff8000000000000ULL); }
 
 // XY::normalize: int / float -> float division, truncation toward zero.

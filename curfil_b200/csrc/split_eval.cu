@@ -794,30 +794,13 @@ level_eval_kernel(EvalArgs a) {
     }
 }
 
-// features per pass-1 work item: two tiles (64 features) were 1 % faster than one, the samples'
-// neighbourhoods serving more features while they are in L1
-constexpr int kStageItemFeatures = 2 * kStageTile;
-
-// bits 0..15 of v spread to the even bit positions (Morton order)
-__device__ __forceinline__ unsigned long long spread_bits(uint32_t v) {
-    unsigned long long x = v & 0xFFFFu;
-    x = (x | (x << 8)) & 0x00FF00FFull;
-    x = (x | (x << 4)) & 0x0F0F0F0Full;
-    x = (x | (x << 2)) & 0x33333333ull;
-    x = (x | (x << 1)) & 0x55555555ull;
-    return x;
-}
-
-// ---- staged bins, pass 1 -------------------------------------------------------------------------
-// Rows of the staged table: row_base[n] + k is sample k of node n. stage_rows_kernel gives every row
-// its sample's position in the level's array and its pixel as the sort key of the pass-1 order: frame
-// by frame, and within a frame in Morton (Z) order of (y, x), so the samples a CTA takes lie in a
-// compact patch and their neighbourhoods overlap in L1 (9 % faster than raster order, whose 256
-// samples span the frame's width).
-__global__ void stage_rows_kernel(const NodeDesc* __restrict__ nodes, const long long* __restrict__ row_base, int M,
+// Sort key of every row (row_base[n] + k is sample k of node n) for the sorted sample copy: node, frame and,
+// within the frame, Morton (Z) order of (y, x), so the samples a CTA takes lie in a compact patch and their
+// neighbourhoods overlap in L1.
+__global__ void order_rows_kernel(const NodeDesc* __restrict__ nodes, const long long* __restrict__ row_base, int M,
                                   long long rows, const Sample* __restrict__ samples, int node_shift,
-                                  int* __restrict__ row_pos, uint8_t* __restrict__ row_label, unsigned long long* __restrict__ pixel_key,
-                                  int* __restrict__ row_ids, int* __restrict__ flip_both) {
+                                  int* __restrict__ row_pos, unsigned long long* __restrict__ pixel_key,
+                                  int* __restrict__ row_ids) {
     const long long r = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (r >= rows) return;
     int lo = 0, hi = M - 1;   // the last node n with row_base[n] <= r
@@ -829,11 +812,9 @@ __global__ void stage_rows_kernel(const NodeDesc* __restrict__ nodes, const long
     const long long p = nodes[lo].start + (r - row_base[lo]);
     const Sample s = samples[p];
     row_pos[r] = static_cast<int>(p);
-    row_label[r] = s.label;
     pixel_key[r] = (static_cast<unsigned long long>(s.image) << 32) | (spread_bits(s.y) << 1) | spread_bits(s.x) |
-                   (node_shift > 0 ? static_cast<unsigned long long>(lo) << node_shift : 0ull);
+                   (static_cast<unsigned long long>(lo) << node_shift);
     row_ids[r] = static_cast<int>(r);
-    if (s.flip == 2) *flip_both = 1;
 }
 
 // The Morton-sorted copy of a level's samples: out[k] is the sample of the k-th row in key order.
@@ -841,78 +822,6 @@ __global__ void gather_sorted_samples_kernel(long long rows, const int* __restri
                                              const Sample* __restrict__ samples, Sample* __restrict__ out) {
     const long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (k < rows) out[k] = samples[row_pos[order[k]]];
-}
-
-struct StageArgs {
-    DsView ds;
-    const Sample* samples;
-    const int* frame_order;   // [rows] rows sorted by frame (stable)
-    const int* row_pos;       // [rows] sample position of each row
-    long long rows;
-    const FeatParams* packs;
-    const float* sorted_thr;  // [F][T]
-    int T;
-    int f_first, n_feat;      // this chunk's features [f_first, f_first + n_feat)
-    uint8_t* out;             // [n_feat / 32 blocks][rows][32]
-};
-
-// One work item = 256 consecutive rows of the frame order x one tile of kStageTile features; items are
-// taken row-block-major, so the resident CTAs evaluate the samples of one or two frames at a time and
-// their corner gathers hit L2. A thread takes one sample through the tile's features (two at a time,
-// their gathers overlapping) and stores each four bins as one word of its row. The bin is that of the
-// fused kernel's feature_bin: the unflipped response for flip 0 and 2, the flipped one for flip 1.
-constexpr int kStageCtasPerSm = 3;   // 4 (56 registers fit) was 5-7 % slower: less L1 per CTA
-
-template <int kPad>
-__global__ void __launch_bounds__(256, kStageCtasPerSm)
-stage_bins_kernel(StageArgs a) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    EvalFeat* s_params = reinterpret_cast<EvalFeat*>(smem);
-    float* s_thr = reinterpret_cast<float*>(smem + sizeof(EvalFeat) * kStageItemFeatures);
-    const int T = a.T;
-    const int TP = kPad ? kPad : T;
-    // (rows padded against the two-way bank conflicts of the search, one word after every 32, were
-    // 2 % slower: the conflicts cost less than the extra index arithmetic)
-    const int TPS = TP;
-    const int W = a.ds.width, H = a.ds.height;
-    const int tiles = (a.n_feat + kStageItemFeatures - 1) / kStageItemFeatures;
-    const long long blocks = (a.rows + 255) / 256;
-    const long long n_items = blocks * tiles;
-    for (long long q = blockIdx.x; q < n_items; q += gridDim.x) {
-        const long long blk = q / tiles;
-        const int j = static_cast<int>(q - blk * tiles);
-        const int fb = j * kStageItemFeatures;
-        const int nf = min(kStageItemFeatures, a.n_feat - fb);
-        const int fg = a.f_first + fb;
-        __syncthreads();   // the previous item's reads of the tile are done
-        for (int i = threadIdx.x; i < nf; i += blockDim.x) s_params[i] = make_eval_feat(a.packs[fg + i]);
-        const float* g_thr = a.sorted_thr + static_cast<long long>(fg) * T;
-        for (int i = threadIdx.x; i < nf * TP; i += blockDim.x) {
-            const int f = i / TP, t = i - f * TP;
-            s_thr[f * TPS + t] = t < T ? g_thr[f * T + t] : INFINITY;
-        }
-        __syncthreads();
-        const long long r = blk * 256 + threadIdx.x;
-        if (r < a.rows) {
-            const int row = a.frame_order[r];
-            const Sample smp = a.samples[a.row_pos[row]];
-            const EvalPixel px = make_eval_pixel(a.ds, smp);
-            const bool flip = smp.flip == 1;
-            uint8_t* seg = a.out + (static_cast<long long>(row) << 5);   // the row's segment of block 0
-            uint32_t acc = 0;
-            for (int f = 0; f < nf; f += 2) {
-                const int b0 = feature_bin(px, W, H, s_params[f], flip, SortedBins<kPad>{s_thr + f * TPS, T});
-                const int b1 =
-                    f + 1 < nf ? feature_bin(px, W, H, s_params[f + 1], flip, SortedBins<kPad>{s_thr + (f + 1) * TPS, T}) : 0;
-                acc |= static_cast<uint32_t>(b0 | (b1 << 8)) << (8 * (f & 3));
-                if ((f & 3) == 2 || f + 2 >= nf) {
-                    const int fw = fb + (f & ~3);   // first feature of the word
-                    *reinterpret_cast<uint32_t*>(seg + ((static_cast<long long>(fw >> 5) * a.rows) << 5) + (fw & 31)) = acc;
-                    acc = 0;
-                }
-            }
-        }
-    }
 }
 
 // One warp per node: the global tie rule over the candidates of the node's items. The lanes stride
@@ -1120,24 +1029,6 @@ void launch_level_eval_a(cf_context* ctx, const EvalArgs& args, int grid, size_t
     }
 }
 
-template <int kPad>
-void launch_stage_bins_t(cf_context* ctx, const StageArgs& a) {
-    const int TP = kPad ? kPad : a.T;
-    const size_t smem = sizeof(EvalFeat) * kStageItemFeatures + sizeof(float) * kStageItemFeatures * TP;
-    set_level_eval_smem(stage_bins_kernel<kPad>, smem, kStageCtasPerSm);
-    const long long items = (a.rows + 255) / 256 * ((a.n_feat + kStageItemFeatures - 1) / kStageItemFeatures);
-    const int grid = static_cast<int>(std::min<long long>(items, static_cast<long long>(ctx->num_sms) * kStageCtasPerSm));
-    launch(ctx, "stage_bins", dim3(grid), dim3(256), smem, stage_bins_kernel<kPad>, a);
-}
-
-void launch_stage_bins(cf_context* ctx, const StageArgs& a) {
-    switch (padded_row(a.T)) {
-        case 32: launch_stage_bins_t<32>(ctx, a); break;
-        case 64: launch_stage_bins_t<64>(ctx, a); break;
-        default: launch_stage_bins_t<0>(ctx, a); break;
-    }
-}
-
 // The level_eval instance for the tuning and threshold count (T <= 31 and 32 <= T <= 63 take the
 // padded branch-free searches).
 void launch_level_eval(cf_context* ctx, const EvalArgs& args, int grid, const EvalTuning& tuning) {
@@ -1293,32 +1184,29 @@ void split_items_into_chunks(const std::vector<int>& node_counts, int chunk, int
     for (int c = n_chunks - 1; c >= 0; c--) chunk_begin[c] = std::min(chunk_begin[c], chunk_begin[c + 1]);
 }
 
-// Rows node by node, and their order sorted by (frame, Morton code), or with by_node by (node, frame,
-// Morton code) for the sorted sample copy of the fused search.
-void LevelEvaluator::stage_order(cf_context* ctx, const DsView& ds, const Sample* samples, const NodeDesc* nodes_dev,
-                                 int M, const std::vector<int>& node_counts, long long rows, bool by_node) {
+void LevelEvaluator::set_row_base(cf_context* ctx, int M, const std::vector<int>& node_counts) {
     h_row_base_.assign(M + 1, 0);
     for (int n = 0; n < M; n++) h_row_base_[n + 1] = h_row_base_[n] + node_counts[n];
     row_base_.reserve(M + 1);
+    CF_CUDA_CHECK(cudaMemcpyAsync(row_base_.get(), h_row_base_.data(), sizeof(long long) * (M + 1),
+                                  cudaMemcpyHostToDevice, ctx->stream));
+}
+
+// Rows node by node, sorted by (node, frame, Morton code) for the sorted sample copy of the fused search.
+void LevelEvaluator::order_rows(cf_context* ctx, const DsView& ds, const Sample* samples, const NodeDesc* nodes_dev,
+                                int M, const std::vector<int>& node_counts, long long rows) {
+    set_row_base(ctx, M, node_counts);
     row_pos_.reserve(rows);
-    row_label_.reserve(rows);
     pixel_key_.reserve(rows);
     pixel_key_sorted_.reserve(rows);
     row_ids_.reserve(rows);
     frame_order_.reserve(rows);
-    CF_CUDA_CHECK(cudaMemcpyAsync(row_base_.get(), h_row_base_.data(), sizeof(long long) * (M + 1),
-                                  cudaMemcpyHostToDevice, ctx->stream));
-    flip_both_.reserve(1);
-    CF_CUDA_CHECK(cudaMemsetAsync(flip_both_.get(), 0, sizeof(int), ctx->stream));
-    int end_bit = 33;   // 32 bits of Morton code, then the frame, then (by_node) the node
+    int end_bit = 33;   // 32 bits of Morton code, then the frame, then the node
     while (end_bit < 64 && (1ull << (end_bit - 32)) < static_cast<unsigned long long>(ds.n)) end_bit++;
-    const int node_shift = by_node ? end_bit : 0;
-    if (by_node)
-        while (end_bit < 64 && (1ull << (end_bit - node_shift)) < static_cast<unsigned long long>(M)) end_bit++;
-    launch(ctx, "stage_rows", dim3(static_cast<unsigned>((rows + 255) / 256)), dim3(256), 0, stage_rows_kernel,
-           nodes_dev, row_base_.get(), M, rows, samples, node_shift, row_pos_.get(), row_label_.get(), pixel_key_.get(),
-           row_ids_.get(),
-           flip_both_.get());
+    const int node_shift = end_bit;
+    while (end_bit < 64 && (1ull << (end_bit - node_shift)) < static_cast<unsigned long long>(M)) end_bit++;
+    launch(ctx, "order_rows", dim3(static_cast<unsigned>((rows + 255) / 256)), dim3(256), 0, order_rows_kernel,
+           nodes_dev, row_base_.get(), M, rows, samples, node_shift, row_pos_.get(), pixel_key_.get(), row_ids_.get());
     size_t temp = 0;
     CF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, temp, pixel_key_.get(), pixel_key_sorted_.get(),
                                                   row_ids_.get(), frame_order_.get(), static_cast<int>(rows), 0,
@@ -1444,28 +1332,20 @@ void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* s
     if (stage) {
         queue_.reserve(n_chunks);
         CF_CUDA_CHECK(cudaMemsetAsync(queue_.get(), 0, sizeof(int) * n_chunks, ctx->stream));
-        stage_order(ctx, ds, samples, nodes_dev, M, node_counts, rows, false);
+        set_row_base(ctx, M, node_counts);
+        row_label_.reserve(rows);
+        flip_both_.reserve(1);
+        stager_.prepare(ctx, ds, samples, nodes_dev, M, row_base_.get(), rows, lf, stage_chunk, n_chunks, row_label_.get(),
+                        flip_both_.get());
         stage_.reserve(stage_bytes);
         args.staged = stage_.get();
         args.staged_rows = rows;
         args.row_label = row_label_.get();
         args.row_base = row_base_.get();
         args.staged_flip_both = flip_both_.get();
-        StageArgs sa;
-        sa.ds = ds;
-        sa.samples = samples;
-        sa.frame_order = frame_order_.get();
-        sa.row_pos = row_pos_.get();
-        sa.rows = rows;
-        sa.packs = lf.packs.get();
-        sa.sorted_thr = lf.sorted_thr.get();
-        sa.T = T;
-        sa.out = stage_.get();
         for (int c = 0; c < n_chunks; c++) {
-            sa.f_first = c * stage_chunk;
-            sa.n_feat = std::min(stage_chunk, F - sa.f_first);
-            launch_stage_bins(ctx, sa);
-            args.staged_f0 = sa.f_first;
+            stager_.run(ctx, ds, samples, lf, c, stage_.get());
+            args.staged_f0 = c * stage_chunk;
             args.order = order_.get() + h_chunk_begin_[c];
             args.n_items = h_chunk_begin_[c + 1] - h_chunk_begin_[c];
             args.queue = queue_.get() + c;
@@ -1482,7 +1362,7 @@ void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* s
         const bool sorted = tuning.sample_order != 0 && rows > 0 && rows < INT_MAX && key_bits <= 64 &&
                             (tuning.sample_order == 2 || frame_bytes > ctx->l2_bytes);
         if (sorted) {
-            stage_order(ctx, ds, samples, nodes_dev, M, node_counts, rows, true);
+            order_rows(ctx, ds, samples, nodes_dev, M, node_counts, rows);
             sorted_samples_.reserve(rows);
             launch(ctx, "gather_sorted_samples", dim3(static_cast<unsigned>((rows + 255) / 256)), dim3(256), 0,
                    gather_sorted_samples_kernel, rows, frame_order_.get(), row_pos_.get(), samples,

@@ -2,16 +2,9 @@
 // per-node kernels.
 #pragma once
 
-#include "features.h"
+#include "stage.h"
 
 namespace cf {
-
-// One open node of a level: its samples are [start, start + count) of the level's sample array.
-struct NodeDesc {
-    long long start;
-    int count;
-    int tree_index;
-};
 
 struct EvalItem {
     int node;
@@ -80,13 +73,12 @@ void plan_level_items(const std::vector<int>& node_counts, int F, const EvalTuni
                       std::vector<EvalItem>& items, std::vector<int>& range, std::vector<int>& order,
                       int chunk_features = 0, int* n_groups = nullptr, int max_groups = 0);
 
-// Staged bins (deep levels): pass 1 computes the threshold bin of every (sample, feature) with the
-// level's samples taken in frame and Morton order, so the resident CTAs gather from one or two frames
-// at a time (L2 hits), and writes it to a byte table of 32-feature blocks, each [row][32 bytes];
-// pass 2 is the split search reading its bins from the table. Rows are the level's samples node by
-// node; the table holds at most stage_max_mb MiB, so a level whose table would be larger runs in
-// feature chunks (multiples of kStageTile features), each pass 1 followed by the items of its features.
-constexpr int kStageTile = 32;   // features per table block
+// Staged bins (deep levels): pass 1 (stage.cu) computes the threshold bin of every (sample, feature) with the
+// level's samples taken in frame and Morton order, so the resident CTAs gather from one or two frames at a
+// time (L2 hits), and writes it to a byte table of 32-feature blocks, each [row][32 bytes]; pass 2 is the
+// split search reading its bins from the table. Rows are the level's samples node by node; the table holds at
+// most stage_max_mb MiB, so a level whose table would be larger runs in feature chunks (multiples of
+// kStageTile features), each pass 1 followed by the items of its features.
 // launch shape of the pass-2 search (level_eval reading staged bins)
 constexpr int kStagedFeatures = 32;           // features per tile at most
 constexpr int kStagedBinsWords = 12288;       // histogram words per CTA
@@ -121,8 +113,10 @@ public:
 
 private:
     void exchange(cf_context* ctx, int n_items);
-    void stage_order(cf_context* ctx, const DsView& ds, const Sample* samples, const NodeDesc* nodes_dev, int M,
-                     const std::vector<int>& node_counts, long long rows, bool by_node);
+    void set_row_base(cf_context* ctx, int M, const std::vector<int>& node_counts);
+    void order_rows(cf_context* ctx, const DsView& ds, const Sample* samples, const NodeDesc* nodes_dev, int M,
+                    const std::vector<int>& node_counts, long long rows);
+    BinStager stager_;                // pass 1 of staged levels
     std::vector<ItemCandidates> h_cands_, h_send_, h_recv_;
     std::vector<int> h_local_order_;
     DevArray<EvalItem> items_;
@@ -139,8 +133,8 @@ private:
     DevArray<uint8_t> row_label_;     // [rows] label of each row's sample
     DevArray<int> flip_both_;         // set when a sample of the level has flip 2
     DevArray<Sample> sorted_samples_; // [rows] the level's samples sorted by (node, frame, Morton code)
-    DevArray<unsigned long long> pixel_key_, pixel_key_sorted_;   // (frame, Morton code of y, x) of each row
-    DevArray<int> row_ids_, frame_order_;   // rows, and rows in pixel order
+    DevArray<unsigned long long> pixel_key_, pixel_key_sorted_;   // (node, frame, Morton code of y, x) of each row
+    DevArray<int> row_ids_, frame_order_;   // rows, and rows in key order
     DevArray<unsigned char> sort_temp_;
     std::vector<long long> h_row_base_;
     std::vector<int> h_chunk_begin_;

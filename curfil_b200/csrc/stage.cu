@@ -1,0 +1,671 @@
+// Pass 1 of the staged split search: every (sample, feature) of a level gets its threshold bin.
+//
+// A response reads eight corners of the sample's integral images, and the lanes of a corner load (one sample
+// each) fall in as many 128-byte lines, so a load of 32 lanes takes 8 cycles of the L1 tag pipe however its
+// data lies: 64 of them per 32 evaluations, 80 with the parameters and the threshold search. That pipe is
+// what bounds the pass (82 % of its peak); the kernel is laid out to need little else:
+//   - 170 instructions per 32 evaluations (feature_bin of eval_fast.cuh: 311). Depth scaling is the
+//     reference's trunc(RN(v / d)): every sample brings a float i with floor(v i) = trunc(RN(v / d)) for every
+//     magnitude v that the level's candidates hold, checked value by value (RN(1 / d) or the next float serves
+//     99.9 % of the depths in whole millimetres; rows of other depths take the general kernel). v i + 2^23
+//     rounded toward zero is then one instruction for two values, and corner offsets are computed as floats
+//     whose bits are the integer;
+//   - a CTA keeps 64 neighbouring samples (frame and Morton order) and walks all features of the chunk, so the
+//     patch that its corners lie in stays in L1 (hit rate 87 %, against 51 % for 256 samples x 64 features).
+// 800 000 samples, 4000 features x 32 thresholds (100 frames 640x480): 49.0 ms before, 31.5 ms after; 8 M samples on
+// 1000 frames: 519 ms, then 320 ms.
+//
+// The bin is the one feature_bin gives, in every case: depth means are compared in float with an error
+// bound and a threshold within it is decided by the exact division; colour sums are exact in double.
+#include <algorithm>
+#include <climits>
+#include <cmath>
+
+#include <cub/device/device_radix_sort.cuh>
+
+#include "eval_fast.cuh"
+#include "stage.h"
+
+namespace cf {
+
+namespace {
+
+using u64 = unsigned long long;
+
+constexpr int kThreads = 512;         // 16 warps: kRows / 32 groups of lanes x 8 unit columns
+constexpr int kCtasPerSm = 2;         // 64 registers; the shared memory left over is L1
+constexpr int kRows = 64;             // samples of a CTA (32: idle lanes of the tag pipe; 128, 256: 2-8 % slower)
+constexpr int kTileFeatures = 128;    // features staged at a time
+constexpr int kMorton = 32;           // key bits below the frame
+constexpr int kGeneralTile = 64;      // features per work item of the general kernel
+constexpr int kGeneralCtasPerSm = 3;
+
+// Floats of a feature's row: eight parameters, +-2^23 with the sign of each offset, then the ascending
+// thresholds padded with +inf: 32 entries serve T <= 31, 36 T = 32, 64 T <= 63.
+constexpr int kRowParams = 12;
+constexpr int kMaxPaddedT = 63;
+int feature_row(int T) { return T < 32 ? kRowParams + 32 : T == 32 ? kRowParams + 36 : kRowParams + 64; }
+
+// Unit lists: depth features, the nine channel pairs, the rest (channels past 2).
+__device__ __forceinline__ int pair_code(const FeatParams& f) {
+    if (f.type == kDepthFeature) return 0;
+    return f.ch1 < 3 && f.ch2 < 3 ? 1 + f.ch1 * 3 + f.ch2 : kStageCodes - 1;
+}
+
+// The largest magnitude a candidate of the level scales by a depth.
+__global__ void stage_reach_kernel(int F, const FeatParams* __restrict__ packs, int* __restrict__ reach) {
+    int m = 1;
+    for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < F; f += gridDim.x * blockDim.x) {
+        const FeatParams p = packs[f];
+        m = max(m, max(max(abs(p.o1x), abs(p.o1y)), max(abs(p.o2x), abs(p.o2y))));
+        m = max(m, max(max(abs(p.r1x), abs(p.r1y)), max(abs(p.r2x), abs(p.r2y))));
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) atomicMax(reach, m);
+}
+
+__global__ void stage_feature_rows_kernel(int F, int T, int row, const FeatParams* __restrict__ packs,
+                                          const float* __restrict__ sorted_thr, float* __restrict__ out) {
+    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    const int f = static_cast<int>(i / row), k = static_cast<int>(i - static_cast<long long>(f) * row);
+    if (f >= (F + kStageUnit - 1) / kStageUnit * kStageUnit) return;
+    float v;
+    if (k < kRowParams) {
+        const FeatParams p = f < F ? packs[f] : FeatParams{};   // whole units: the rows past F hold zeros
+        const int8_t par[8] = {p.o1x, p.o1y, p.o2x, p.o2y, p.r1x, p.r1y, p.r2x, p.r2y};
+        v = k < 8 ? static_cast<float>(par[k]) : par[k - 8] < 0 ? -8388608.0f : 8388608.0f;
+    } else {
+        const int t = k - kRowParams;
+        v = t < T && f < F ? sorted_thr[static_cast<long long>(f) * T + t] : INFINITY;
+    }
+    out[i] = v;
+}
+
+// One CTA per feature chunk: the 8-feature blocks of every code (a block with features of several codes is
+// listed in each, with the mask of its features).
+__global__ void __launch_bounds__(256)
+stage_units_kernel(int F, int chunk, int cap, const FeatParams* __restrict__ packs, uint32_t* __restrict__ units,
+                   int* __restrict__ unit_count) {
+    __shared__ int s_n[kStageCodes];
+    const int f0 = blockIdx.x * chunk, n = min(chunk, F - f0);
+    if (threadIdx.x < kStageCodes) s_n[threadIdx.x] = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int blocks = (n + kStageUnit - 1) / kStageUnit;
+    uint32_t* mine = units + static_cast<long long>(blockIdx.x) * kStageCodes * cap;
+    if (threadIdx.x < 32) {   // one warp, in block order
+        for (int b0 = 0; b0 < blocks; b0 += 32) {
+            const int b = b0 + lane;
+            u64 codes = ~0ull;   // 4 bits per feature, 15: none
+            for (int j = 0; j < kStageUnit; j++) {
+                const int f = b * kStageUnit + j;
+                const u64 c = b < blocks && f < n ? pair_code(packs[f0 + f]) : 15;
+                codes = (codes & ~(15ull << (4 * j))) | (c << (4 * j));
+            }
+            for (int c = 0; c < kStageCodes; c++) {
+                uint32_t mask = 0;
+                for (int j = 0; j < kStageUnit; j++)
+                    if (((codes >> (4 * j)) & 15ull) == static_cast<u64>(c)) mask |= 1u << j;
+                const unsigned bal = __ballot_sync(0xffffffffu, mask != 0);
+                const int at = s_n[c] + __popc(bal & ((1u << lane) - 1u));
+                if (mask) mine[c * cap + at] = static_cast<uint32_t>(b) << 8 | mask;
+                __syncwarp();
+                if (lane == 0) s_n[c] += __popc(bal);
+                __syncwarp();
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < kStageCodes) unit_count[blockIdx.x * kStageCodes + threadIdx.x] = s_n[threadIdx.x];
+}
+
+// A float i with floor(v i) = trunc(RN(v / d)) for v = 1 .. most (RN(1 / d) or the next float), or 0.
+__device__ __forceinline__ float checked_reciprocal(float d, int most) {
+    float inv = __frcp_rn(d);
+    for (int k = 0; k < 2; k++) {
+        bool same = true;
+        for (int v = 1; v <= most && same; v++) {
+            const float f = __uint2float_rn(v);
+            same = __fmaf_rz(f, inv, 8388608.0f) == __fadd_rz(__fdiv_rn(f, d), 8388608.0f);
+        }
+        if (same) return inv;
+        inv = __uint_as_float(__float_as_uint(inv) + 1u);
+    }
+    return 0.0f;
+}
+
+// Rows of the table: row_base[n] + k is sample k of node n. Pass 1 takes them frame by frame and within a
+// frame in Morton (Z) order of (y, x), so that the rows a CTA takes lie in a compact patch; rows without a
+// checked reciprocal come last, in the same order.
+__global__ void stage_rows_kernel(const NodeDesc* __restrict__ nodes, const long long* __restrict__ row_base, int M,
+                                  long long rows, const Sample* __restrict__ samples, const int* __restrict__ reach,
+                                  int padded, int frame_bits, int* __restrict__ row_pos, uint8_t* __restrict__ row_label,
+                                  u64* __restrict__ key, int* __restrict__ row_ids, float* __restrict__ row_inv,
+                                  int* __restrict__ flip_both) {
+    const long long r = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    if (r >= rows) return;
+    int lo = 0, hi = M - 1;   // the last node n with row_base[n] <= r
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (row_base[mid] <= r) lo = mid;
+        else hi = mid - 1;
+    }
+    const long long p = nodes[lo].start + (r - row_base[lo]);
+    const Sample s = samples[p];
+    row_pos[r] = static_cast<int>(p);
+    row_label[r] = s.label;
+    row_ids[r] = static_cast<int>(r);
+    if (s.flip == 2) *flip_both = 1;
+    float inv = 1.0f;   // an invalid depth scales nothing
+    if (s.depth > 0.0f)
+        inv = s.depth >= 1e-3f && s.depth <= 1e6f ? checked_reciprocal(s.depth, *reach) : 0.0f;   // |v / d| < 2^18
+    if (!padded) inv = 0.0f;
+    row_inv[r] = inv;
+    key[r] = (inv == 0.0f ? 1ull << (kMorton + frame_bits) : 0ull) | static_cast<u64>(s.image) << kMorton |
+             spread_bits(s.y) << 1 | spread_bits(s.x);
+}
+
+// The rows in key order, and where the rows without a checked reciprocal begin.
+__global__ void stage_list_kernel(long long rows, int general_bit, const u64* __restrict__ key,
+                                  const int* __restrict__ order, const int* __restrict__ row_pos,
+                                  const Sample* __restrict__ samples, const float* __restrict__ row_inv,
+                                  int* __restrict__ general_begin, StageSample* __restrict__ out) {
+    const long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    if (k >= rows) return;
+    const int row = order[k];
+    const Sample s = samples[row_pos[row]];
+    StageSample o;
+    o.x = s.x;
+    o.y = s.y;
+    o.image = s.image;
+    o.row = static_cast<uint32_t>(row) | (s.flip == 1 ? 0x80000000u : 0u);
+    o.inv_d = s.depth > 0.0f ? row_inv[row] : 0.0f;
+    out[k] = o;
+    const bool general = key[k] >> general_bit;
+    if (general && (k == 0 || !(key[k - 1] >> general_bit))) *general_begin = static_cast<int>(k);
+    if (!general && k == rows - 1) *general_begin = static_cast<int>(rows);
+}
+
+struct StageArgs {
+    DsView ds;
+    const Sample* samples;    // the level's samples
+    const int* row_pos;
+    long long rows;
+    const StageSample* list;
+    const int* order;
+    const int* general_begin;
+    const FeatParams* packs;
+    const float* sorted_thr;  // [F][T]
+    const float* feature_rows;
+    int T;
+    int f_first, n_feat;      // the chunk's features [f_first, f_first + n_feat)
+    const uint32_t* units;    // [codes][cap]
+    const int* unit_count;    // [codes]
+    int cap;
+    int parts;                // work items per block of rows
+    uint8_t* out;             // [n_feat / 32 blocks][rows][32]
+};
+
+__device__ __forceinline__ uint8_t* bin_place(const StageArgs& a, int g, long long row) {
+    return a.out + (((g >> 5) * a.rows + row) << 5) + (g & 31);
+}
+
+// ---- two floats per instruction -----------------------------------------------------------------
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ u64 fma2_rz(u64 a, u64 b, u64 c) {
+    u64 r;
+    asm("fma.rz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+    u64 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 sub2(u64 a, u64 b) {
+    u64 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(u64 v) {
+    float2 r;
+    unpack_f2(v, r.x, r.y);
+    return r;
+}
+
+// What a lane holds of its sample, and of the frame for the features at hand.
+struct Lane {
+    u64 pos;        // (x, y)
+    u64 inv;        // the sample's checked reciprocal, twice
+    u64 side;       // (1 or -1 for a flipped response, 1)
+};
+
+// Bytes of an element and of a row and the first bytes of the planes of box 1 and box 2, as multiples of the
+// smallest denormal: such a float's bits are the integer, up to 2^24, so offsets need no conversion.
+struct FrameView {
+    float xmax, ymax, size, pitch, base1, base2;
+};
+
+// trunc(RN(v / d)) of two parameters; big = 2^23 with each value's sign
+__device__ __forceinline__ u64 scale2(u64 v, const Lane& l, u64 big) {
+    return sub2(fma2_rz(v, l.inv, big), big);
+}
+
+// Thresholds below v of a padded row (32 entries serve T <= 31, 36 T = 32, 64 T <= 63): halving, on a byte
+// offset so that a step is a read, a compare and an addition.
+template <int kRow>
+__device__ __forceinline__ int row_below(const float* t, float v) {
+    const char* at = reinterpret_cast<const char*>(t);
+    auto entry = [&](int k) { return *reinterpret_cast<const float*>(at + 4 * k); };
+    constexpr int kEntries = kRow - kRowParams;
+    if (kEntries == 64) {
+        if (t[31] < v) at += 128;
+    }
+    if (entry(15) < v) at += 64;
+    if (entry(7) < v) at += 32;
+    if (entry(3) < v) at += 16;
+    if (entry(1) < v) at += 8;
+    if (entry(0) < v) at += 4;
+    const int k = static_cast<int>(at - reinterpret_cast<const char*>(t)) >> 2;
+    return kEntries == 36 ? k + (t[31] < v ? 1 : 0) : k;
+}
+
+// The two boxes of one feature: byte offsets of their corners in the sample's frame, and whether both
+// lie inside it.
+struct Corners {
+    int ul1, ur1, ll1, lr1, ul2, ur2, ll2, lr2;
+    bool in;
+};
+
+__device__ __forceinline__ Corners corners(const Lane& l, const float* row, const FrameView& p) {
+    const ulonglong2 o = *reinterpret_cast<const ulonglong2*>(row);          // o1, o2
+    const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(row + 4);      // r1, r2
+    const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(row + 8);      // 2^23 with the offsets' signs
+    const u64 big = pack_f2(8388608.0f, 8388608.0f);
+    const u64 c1 = fma2(scale2(o.x, l, b.x), l.side, l.pos);
+    const u64 c2 = fma2(scale2(o.y, l, b.y), l.side, l.pos);
+    const float2 g1 = unpack2(scale2(g.x, l, big)), g2 = unpack2(scale2(g.y, l, big));
+    const float w1 = fmaxf(g1.x, 1.0f), h1 = fmaxf(g1.y, 1.0f), w2 = fmaxf(g2.x, 1.0f), h2 = fmaxf(g2.y, 1.0f);
+    const u64 s1 = pack_f2(w1, h1), s2 = pack_f2(w2, h2);
+    const float2 lo1 = unpack2(sub2(c1, s1)), hi1 = unpack2(add2(c1, s1));
+    const float2 lo2 = unpack2(sub2(c2, s2)), hi2 = unpack2(add2(c2, s2));
+    Corners k;
+    k.in = fminf(fminf(lo1.x, lo1.y), fminf(lo2.x, lo2.y)) >= 0.0f && fmaxf(hi1.x, hi2.x) <= p.xmax &&
+           fmaxf(hi1.y, hi2.y) <= p.ymax;
+    const float l1 = fmaf(lo1.x, p.size, p.base1), r1 = fmaf(hi1.x, p.size, p.base1);
+    const float l2 = fmaf(lo2.x, p.size, p.base2), r2 = fmaf(hi2.x, p.size, p.base2);
+    k.ul1 = __float_as_int(fmaf(lo1.y, p.pitch, l1));
+    k.ur1 = __float_as_int(fmaf(lo1.y, p.pitch, r1));
+    k.ll1 = __float_as_int(fmaf(hi1.y, p.pitch, l1));
+    k.lr1 = __float_as_int(fmaf(hi1.y, p.pitch, r1));
+    k.ul2 = __float_as_int(fmaf(lo2.y, p.pitch, l2));
+    k.ur2 = __float_as_int(fmaf(lo2.y, p.pitch, r2));
+    k.ll2 = __float_as_int(fmaf(hi2.y, p.pitch, l2));
+    k.lr2 = __float_as_int(fmaf(hi2.y, p.pitch, r2));
+    return k;
+}
+
+template <typename V>
+__device__ __forceinline__ V frame_at(const unsigned char* frame, int offset) {
+    return __ldg(reinterpret_cast<const V*>(frame + offset));
+}
+
+// The box sums and counts of a depth feature, and whether its bin still has to be found from them (a threshold
+// lies within the error bound, or a count is outside [1, 2^23)).
+struct DepthBoxes {
+    int s1, n1, s2, n2;
+    bool open;
+};
+
+template <int kRow>
+__device__ __forceinline__ int depth_bin(const Lane& l, const float* row, const unsigned char* frame,
+                                                const FrameView& p, int T, DepthBoxes& box) {
+    const Corners k = corners(l, row, p);
+    int2 ul1 = make_int2(0, 0), ur1 = ul1, ll1 = ul1, lr1 = ul1, ul2 = ul1, ur2 = ul1, ll2 = ul1, lr2 = ul1;
+    if (k.in) {
+        ul1 = frame_at<int2>(frame, k.ul1), ur1 = frame_at<int2>(frame, k.ur1);
+        ll1 = frame_at<int2>(frame, k.ll1), lr1 = frame_at<int2>(frame, k.lr1);
+        ul2 = frame_at<int2>(frame, k.ul2), ur2 = frame_at<int2>(frame, k.ur2);
+        ll2 = frame_at<int2>(frame, k.ll2), lr2 = frame_at<int2>(frame, k.lr2);
+    }
+    auto sum = [](int lr, int ur, int ul, int ll) {
+        return static_cast<int>(static_cast<uint32_t>(lr) - static_cast<uint32_t>(ur) + static_cast<uint32_t>(ul) - static_cast<uint32_t>(ll));
+    };
+    box.s1 = sum(lr1.x, ur1.x, ul1.x, ll1.x);
+    box.n1 = sum(lr1.y, ur1.y, ul1.y, ll1.y);
+    box.s2 = sum(lr2.x, ur2.x, ul2.x, ll2.x);
+    box.n2 = sum(lr2.y, ur2.y, ul2.y, ll2.y);
+    const float n1 = __int_as_float(0x4B000000 + box.n1) - 8388608.0f;
+    const float n2 = __int_as_float(0x4B000000 + box.n2) - 8388608.0f;
+    float i1, i2;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(i1) : "f"(n1));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(i2) : "f"(n2));
+    // means in mm: the conversion is within 2^-24, the reciprocal within 2^-23, the products, the difference,
+    // 0.001f and the last rounding within 2^-24 each: the response in metres is within 4.1e-10 (a + b) of the
+    // exact one, and 5e-10 (a + b) bounds it
+    const float a = static_cast<float>(box.s1) * i1, b = static_cast<float>(box.s2) * i2;
+    const float delta = fmaf(fabsf(a) + fabsf(b), 5e-10f, 1e-30f);
+    const float r = a - b;
+    const float* t = row + kRowParams;
+    const int bin = row_below<kRow>(t, fmaf(r, 0.001f, -delta));
+    const bool clear = t[bin] > fmaf(r, 0.001f, delta);
+    const bool some = k.in && box.n1 != 0 && box.n2 != 0;
+    const bool plain = (static_cast<uint32_t>(box.n1 - 1) | static_cast<uint32_t>(box.n2 - 1)) < 0x7FFFFFu;
+    box.open = some && !(clear && plain);
+    return some ? bin : T;
+}
+
+template <int kRow>
+__device__ __noinline__ int open_bin(int s1, int n1, int s2, int n2, const float* t) {
+    return row_below<kRow>(t, __double2float_ru(exact_depth_response(s1, n1, s2, n2)));
+}
+
+template <int kRow>
+__device__ __forceinline__ int color_bin(const Lane& l, const float* row, const unsigned char* frame,
+                                                const FrameView& p, int T) {
+    const Corners k = corners(l, row, p);
+    float ul1 = 0, ur1 = 0, ll1 = 0, lr1 = 0, ul2 = 0, ur2 = 0, ll2 = 0, lr2 = 0;
+    if (k.in) {
+        ul1 = frame_at<float>(frame, k.ul1), ur1 = frame_at<float>(frame, k.ur1);
+        ll1 = frame_at<float>(frame, k.ll1), lr1 = frame_at<float>(frame, k.lr1);
+        ul2 = frame_at<float>(frame, k.ul2), ur2 = frame_at<float>(frame, k.ur2);
+        ll2 = frame_at<float>(frame, k.ll2), lr2 = frame_at<float>(frame, k.lr2);
+    }
+    const double A = __dadd_rn(__dsub_rn(lr1, ur1), __dsub_rn(ul1, ll1));
+    const double B = __dadd_rn(__dsub_rn(lr2, ur2), __dsub_rn(ul2, ll2));
+    const double r = __dsub_rn(A, B);   // NaN if a corner is
+    const int bin = row_below<kRow>(row + kRowParams, __double2float_ru(r));
+    return k.in && !isnan(r) ? bin : T;
+}
+
+// One work item = 64 rows of the list x the chunk's features (in `parts` parts where there are few rows). The
+// lanes of a warp keep 32 samples, the CTA's eight unit columns share each group of samples and take the
+// tile's 8-feature units in turn, two features of a unit at a time so that their gathers overlap, and store a
+// unit's bins as one 8-byte word.
+template <int kRow>
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
+stage_gather_kernel(const __grid_constant__ StageArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    float* rows = reinterpret_cast<float*>(smem);
+    constexpr int kUnits = kTileFeatures / kStageUnit;
+    constexpr int kGroups = kRows / 32, kColumns = kThreads / kRows;
+    __shared__ uint32_t s_unit[kUnits];
+    const int T = a.T;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int column = warp / kGroups;
+    int n_units = 0;
+    for (int c = 0; c < kStageCodes - 1; c++) n_units += a.unit_count[c];
+    const int tiles = (n_units + kUnits - 1) / kUnits;
+    const long long end = *a.general_begin;
+    const long long items = (end + kRows - 1) / kRows * a.parts;
+    for (long long item = blockIdx.x; item < items; item += gridDim.x) {
+        const long long blk = item / a.parts;
+        const int part = static_cast<int>(item - blk * a.parts);
+        const long long k = blk * kRows + (warp % kGroups) * 32 + lane;
+        const bool have = k < end;
+        const StageSample s = a.list[have ? k : end - 1];
+        const bool valid = s.inv_d > 0.0f;
+        Lane l;
+        const float inv = valid ? s.inv_d : 1.0f;
+        l.pos = pack_f2(static_cast<float>(s.x), static_cast<float>(s.y));
+        l.inv = pack_f2(inv, inv);
+        l.side = pack_f2(s.row >> 31 ? -1.0f : 1.0f, 1.0f);
+        const int row = static_cast<int>(s.row & 0x7FFFFFFFu);
+        const unsigned char* depth = reinterpret_cast<const unsigned char*>(a.ds.depth + s.image * a.ds.plane);
+        const unsigned char* color = reinterpret_cast<const unsigned char*>(a.ds.color + s.image * 3ll * a.ds.plane);
+        FrameView view;
+        view.xmax = static_cast<float>(a.ds.width - 1);
+        view.ymax = static_cast<float>(a.ds.height - 1);
+        const int plane = static_cast<int>(a.ds.plane) * 4;
+        for (int j = tiles * part / a.parts; j < tiles * (part + 1) / a.parts; j++) {
+            const int nu = min(kUnits, n_units - j * kUnits);
+            __syncthreads();   // the previous tile is read
+            if (static_cast<int>(threadIdx.x) < nu) {
+                int v = j * kUnits + threadIdx.x, c = 0;
+                while (v >= a.unit_count[c]) v -= a.unit_count[c++];
+                s_unit[threadIdx.x] = a.units[c * a.cap + v] | static_cast<uint32_t>(c) << 28;
+            }
+            __syncthreads();
+            constexpr int kQuads = kStageUnit * kRow / 4;
+            for (int i = threadIdx.x; i < nu * kQuads; i += kThreads) {
+                const int u = i / kQuads;
+                const int f0 = a.f_first + static_cast<int>(s_unit[u] >> 8 & 0xFFFFFu) * kStageUnit;
+                reinterpret_cast<float4*>(rows)[i] = __ldg(
+                    reinterpret_cast<const float4*>(a.feature_rows + static_cast<long long>(f0) * kRow) + (i - u * kQuads));
+            }
+            __syncthreads();
+            for (int u = column; u < nu; u += kColumns) {
+                const uint32_t unit = s_unit[u];
+                const uint32_t mask = unit & 255u;
+                const int code = unit >> 28;
+                const float* r = rows + u * kStageUnit * kRow;
+                uint32_t lo = 0, hi = 0;
+                if (code == 0) {
+                    view.size = __int_as_float(8);
+                    view.pitch = __int_as_float(8 * a.ds.width);
+                    view.base1 = view.base2 = 0.0f;
+                    for (int i = 0; i < kStageUnit; i += 2, r += 2 * kRow) {
+                        DepthBoxes x0, x1;
+                        int b0 = depth_bin<kRow>(l, r, depth, view, T, x0);
+                        int b1 = depth_bin<kRow>(l, r + kRow, depth, view, T, x1);
+                        if (x0.open) b0 = open_bin<kRow>(x0.s1, x0.n1, x0.s2, x0.n2, r + kRowParams);
+                        if (x1.open) b1 = open_bin<kRow>(x1.s1, x1.n1, x1.s2, x1.n2, r + kRow + kRowParams);
+                        lo = __byte_perm(lo, hi, 0x5432);                        // (hi, lo) moves down two bytes
+                        hi = __byte_perm(hi, __byte_perm(b0, b1, 0x0040), 0x5432);
+                    }
+                } else {
+                    view.size = __int_as_float(4);
+                    view.pitch = __int_as_float(4 * a.ds.width);
+                    view.base1 = __int_as_float((code - 1) / 3 * plane);
+                    view.base2 = __int_as_float((code - 1) % 3 * plane);
+                    for (int i = 0; i < kStageUnit; i += 2, r += 2 * kRow) {
+                        const int b0 = color_bin<kRow>(l, r, color, view, T);
+                        const int b1 = color_bin<kRow>(l, r + kRow, color, view, T);
+                        lo = __byte_perm(lo, hi, 0x5432);
+                        hi = __byte_perm(hi, __byte_perm(b0, b1, 0x0040), 0x5432);
+                    }
+                }
+                if (!valid) lo = hi = static_cast<uint32_t>(T) * 0x01010101u;
+                if (have) {
+                    uint8_t* to = bin_place(a, static_cast<int>(unit >> 8 & 0xFFFFFu) * kStageUnit, row);
+                    if (mask == 255u) {
+                        *reinterpret_cast<uint2*>(to) = make_uint2(lo, hi);
+                    } else {
+                        const u64 word = static_cast<u64>(hi) << 32 | lo;
+                        for (int i = 0; i < kStageUnit; i++)
+                            if (mask >> i & 1u) to[i] = static_cast<uint8_t>(word >> (8 * i));
+                    }
+                }
+            }
+        }
+    }
+}
+
+// feature_bin itself: rows without a checked reciprocal with all features, then all rows with the features of
+// other channels. One work item = 256 consecutive rows of the list x up to kGeneralTile features.
+template <int kPad>
+__global__ void __launch_bounds__(256, kGeneralCtasPerSm)
+stage_general_kernel(const __grid_constant__ StageArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    EvalFeat* s_params = reinterpret_cast<EvalFeat*>(smem);
+    float* s_thr = reinterpret_cast<float*>(smem + sizeof(EvalFeat) * kGeneralTile);
+    __shared__ uint32_t s_unit[kGeneralTile / kStageUnit];
+    constexpr int kUnits = kGeneralTile / kStageUnit;
+    const int T = a.T;
+    const int TP = kPad ? kPad : T;
+    const int W = a.ds.width, H = a.ds.height;
+    for (int seg = 0; seg < 2; seg++) {
+        const int code_a = seg == 0 ? 0 : kStageCodes - 1, code_b = seg == 0 ? kStageCodes - 1 : kStageCodes;
+        int n_units = 0;
+        for (int c = code_a; c < code_b; c++) n_units += a.unit_count[c];
+        const long long begin = seg == 0 ? *a.general_begin : 0;
+        const int tiles = (n_units + kUnits - 1) / kUnits;
+        const long long items = (a.rows - begin + 255) / 256 * tiles;
+        for (long long q = blockIdx.x; q < items; q += gridDim.x) {
+            const long long blk = q / tiles;
+            const int j = static_cast<int>(q - blk * tiles);
+            const int nu = min(kUnits, n_units - j * kUnits);
+            __syncthreads();   // the previous item's reads of the tile are done
+            if (static_cast<int>(threadIdx.x) < nu) {
+                int v = j * kUnits + threadIdx.x, c = code_a;
+                while (v >= a.unit_count[c]) v -= a.unit_count[c++];
+                s_unit[threadIdx.x] = a.units[c * a.cap + v];
+            }
+            __syncthreads();
+            for (int i = threadIdx.x; i < nu * kStageUnit; i += blockDim.x) {
+                const int g = static_cast<int>(s_unit[i / kStageUnit] >> 8) * kStageUnit + i % kStageUnit;
+                if (g < a.n_feat) s_params[i] = make_eval_feat(a.packs[a.f_first + g]);
+            }
+            for (int i = threadIdx.x; i < nu * kStageUnit * TP; i += blockDim.x) {
+                const int f = i / TP, t = i - f * TP;
+                const int g = static_cast<int>(s_unit[f / kStageUnit] >> 8) * kStageUnit + f % kStageUnit;
+                s_thr[i] = t < T && g < a.n_feat ? a.sorted_thr[static_cast<long long>(a.f_first + g) * T + t] : INFINITY;
+            }
+            __syncthreads();
+            const long long k = begin + blk * 256 + threadIdx.x;
+            if (k >= a.rows) continue;
+            const int row = a.order[k];
+            const Sample smp = a.samples[a.row_pos[row]];
+            const EvalPixel px = make_eval_pixel(a.ds, smp);
+            const bool flip = smp.flip == 1;
+            for (int u = 0; u < nu; u++) {
+                const uint32_t unit = s_unit[u];
+                const uint32_t mask = unit & 255u;
+                uint8_t* to = bin_place(a, static_cast<int>(unit >> 8) * kStageUnit, row);
+                u64 word = 0;
+                for (int i = 0; i < kStageUnit; i += 2) {
+                    const int f = u * kStageUnit + i;
+                    int b0 = 0, b1 = 0;
+                    if (mask >> i & 1u) b0 = feature_bin(px, W, H, s_params[f], flip, SortedBins<kPad>{s_thr + f * TP, T});
+                    if (mask >> i & 2u)
+                        b1 = feature_bin(px, W, H, s_params[f + 1], flip, SortedBins<kPad>{s_thr + (f + 1) * TP, T});
+                    word |= static_cast<u64>(static_cast<uint32_t>(b0 | b1 << 8)) << (8 * i);
+                }
+                if (mask == 255u) {
+                    *reinterpret_cast<u64*>(to) = word;
+                } else {
+                    for (int i = 0; i < kStageUnit; i++)
+                        if (mask >> i & 1u) to[i] = static_cast<uint8_t>(word >> (8 * i));
+                }
+            }
+        }
+    }
+}
+
+template <typename K>
+void set_smem(K kernel, size_t smem, int ctas) {
+    // the carveout that just holds the resident CTAs; the rest of the unified memory caches the gathers
+    const double need = ctas * (smem + 2048.0);
+    CF_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    CF_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                       std::min(100, static_cast<int>(std::ceil(100.0 * need / (228.0 * 1024))))));
+}
+
+template <int kPad>
+void launch_general(cf_context* ctx, const char* name, const StageArgs& a) {
+    const int TP = kPad ? kPad : a.T;
+    const size_t smem = sizeof(EvalFeat) * kGeneralTile + sizeof(float) * kGeneralTile * TP;
+    set_smem(stage_general_kernel<kPad>, smem, kGeneralCtasPerSm);
+    launch(ctx, name, dim3(ctx->num_sms * kGeneralCtasPerSm), dim3(256), smem, stage_general_kernel<kPad>, a);
+}
+
+}  // namespace
+
+void BinStager::prepare(cf_context* ctx, const DsView& ds, const Sample* samples, const NodeDesc* nodes_dev, int M,
+                        const long long* row_base_dev, long long rows, const LevelFeatures& lf, int chunk,
+                        int n_chunks, uint8_t* row_label, int* flip_both) {
+    rows_ = rows;
+    chunk_ = chunk;
+    cap_ = (chunk + kStageUnit - 1) / kStageUnit;
+    // the padded threshold rows serve T <= 63, the float offsets frames of up to 2^24 bytes of depth integral
+    // (1280x960: 9.8 MB); otherwise every row takes the general kernel
+    padded_ = lf.T <= kMaxPaddedT && ds.plane * 12 <= (1ll << 24);
+    int frame_bits = 1;
+    while ((1ll << frame_bits) < ds.n) frame_bits++;
+    cudaStream_t st = ctx->stream;
+    reach_.reserve(1);
+    CF_CUDA_CHECK(cudaMemsetAsync(reach_.get(), 0, sizeof(int), st));
+    launch(ctx, "stage_plan", dim3(std::min(64, (lf.F + 255) / 256)), dim3(256), 0, stage_reach_kernel, lf.F, lf.packs.get(),
+           reach_.get());
+    if (padded_) {
+        const int row = feature_row(lf.T);
+        const long long n = (lf.F + kStageUnit - 1ll) / kStageUnit * kStageUnit * row;
+        rows_f_.reserve(n);
+        launch(ctx, "stage_plan", dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, stage_feature_rows_kernel,
+               lf.F, lf.T, row, lf.packs.get(), lf.sorted_thr.get(), rows_f_.get());
+    }
+    units_.reserve(static_cast<size_t>(n_chunks) * kStageCodes * cap_);
+    unit_count_.reserve(static_cast<size_t>(n_chunks) * kStageCodes);
+    launch(ctx, "stage_plan", dim3(n_chunks), dim3(32), 0, stage_units_kernel, lf.F, chunk, cap_, lf.packs.get(),
+           units_.get(), unit_count_.get());
+    row_pos_.reserve(rows);
+    row_ids_.reserve(rows);
+    row_inv_.reserve(rows);
+    key_.reserve(rows);
+    key_sorted_.reserve(rows);
+    order_.reserve(rows);
+    list_.reserve(rows);
+    general_begin_.reserve(1);
+    CF_CUDA_CHECK(cudaMemsetAsync(flip_both, 0, sizeof(int), st));
+    const dim3 grid(static_cast<unsigned>((rows + 255) / 256));
+    launch(ctx, "stage_rows", grid, dim3(256), 0, stage_rows_kernel, nodes_dev, row_base_dev, M, rows, samples,
+           static_cast<const int*>(reach_.get()), padded_ ? 1 : 0, frame_bits, row_pos_.get(), row_label, key_.get(),
+           row_ids_.get(), row_inv_.get(), flip_both);
+    const int general_bit = kMorton + frame_bits;
+    size_t temp = 0;
+    CF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, temp, key_.get(), key_sorted_.get(), row_ids_.get(),
+                                                  order_.get(), static_cast<int>(rows), 0, general_bit + 1, st));
+    sort_temp_.reserve(temp);
+    CF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(sort_temp_.get(), temp, key_.get(), key_sorted_.get(),
+                                                  row_ids_.get(), order_.get(), static_cast<int>(rows), 0,
+                                                  general_bit + 1, st));
+    launch(ctx, "stage_rows", grid, dim3(256), 0, stage_list_kernel, rows, general_bit,
+           static_cast<const u64*>(key_sorted_.get()), order_.get(), row_pos_.get(), samples, row_inv_.get(),
+           general_begin_.get(), list_.get());
+}
+
+void BinStager::run(cf_context* ctx, const DsView& ds, const Sample* samples, const LevelFeatures& lf, int c,
+                    uint8_t* out) {
+    StageArgs a;
+    a.ds = ds;
+    a.samples = samples;
+    a.row_pos = row_pos_.get();
+    a.rows = rows_;
+    a.list = list_.get();
+    a.order = order_.get();
+    a.general_begin = general_begin_.get();
+    a.packs = lf.packs.get();
+    a.sorted_thr = lf.sorted_thr.get();
+    a.feature_rows = rows_f_.get();
+    a.T = lf.T;
+    a.f_first = c * chunk_;
+    a.n_feat = std::min(chunk_, lf.F - a.f_first);
+    a.units = units_.get() + static_cast<size_t>(c) * kStageCodes * cap_;
+    a.unit_count = unit_count_.get() + c * kStageCodes;
+    a.cap = cap_;
+    a.out = out;
+    if (padded_) {
+        auto kernel = lf.T < 32 ? stage_gather_kernel<kRowParams + 32>
+                                : lf.T == 32 ? stage_gather_kernel<kRowParams + 36> : stage_gather_kernel<kRowParams + 64>;
+        const size_t smem = sizeof(float) * kTileFeatures * feature_row(lf.T);
+        set_smem(kernel, smem, kCtasPerSm);
+        // few rows: their features in parts, for about eight work items per resident CTA
+        const long long blocks = (rows_ + kRows - 1) / kRows, slots = static_cast<long long>(ctx->num_sms) * kCtasPerSm;
+        const int tiles = (a.n_feat + kTileFeatures - 1) / kTileFeatures;
+        a.parts = static_cast<int>(std::max<long long>(1, std::min<long long>(tiles, 8 * slots / blocks)));
+        launch(ctx, "stage_bins", dim3(static_cast<unsigned>(std::min(slots, blocks * a.parts))), dim3(kThreads), smem,
+               kernel, a);
+    }
+    const char* name = padded_ ? "stage_general" : "stage_bins";
+    switch (padded_row(lf.T)) {
+        case 32: launch_general<32>(ctx, name, a); break;
+        case 64: launch_general<64>(ctx, name, a); break;
+        default: launch_general<0>(ctx, name, a); break;
+    }
+}
+
+}  // namespace cf

@@ -1,0 +1,53 @@
+// Pass 1 of the staged split search: the threshold bin of every (sample, feature) of a level.
+#pragma once
+
+#include "features.h"
+
+namespace cf {
+
+// One open node of a level: its samples are [start, start + count) of the level's sample array.
+struct NodeDesc {
+    long long start;
+    int count;
+    int tree_index;
+};
+
+constexpr int kStageTile = 32;     // features per table block
+constexpr int kStageUnit = 8;      // features a lane takes at a time
+constexpr int kStageCodes = 11;    // unit lists: depth, the nine colour channel pairs, the rest
+
+// One row of the pass-1 order.
+struct __align__(16) StageSample {
+    uint16_t x, y;
+    uint32_t image;
+    uint32_t row;                  // table row; bit 31: the flipped response is wanted
+    float inv_d;                   // checked reciprocal of the depth; 0: invalid depth, every response is NaN
+};
+
+class BinStager {
+public:
+    // Orders the level's rows (row_base[n] + k is sample k of node n) and lays out the candidates of its
+    // n_chunks feature chunks of `chunk` features.
+    void prepare(cf_context* ctx, const DsView& ds, const Sample* samples, const NodeDesc* nodes_dev, int M,
+                 const long long* row_base_dev, long long rows, const LevelFeatures& lf, int chunk, int n_chunks,
+                 uint8_t* row_label, int* flip_both);
+    // The bins of chunk c: feature f of the chunk and row r at out[((f / 32) * rows + r) * 32 + f % 32].
+    void run(cf_context* ctx, const DsView& ds, const Sample* samples, const LevelFeatures& lf, int c, uint8_t* out);
+
+private:
+    long long rows_ = 0;
+    int chunk_ = 0, cap_ = 0;
+    bool padded_ = false;          // the level's thresholds and frames suit the gather kernel
+    DevArray<unsigned long long> key_, key_sorted_;
+    DevArray<int> row_pos_, row_ids_, order_;
+    DevArray<float> row_inv_;      // [rows] checked reciprocal of each row's depth, 0 if there is none
+    DevArray<StageSample> list_;   // [rows] in pass-1 order
+    DevArray<int> general_begin_;  // first list position without a checked reciprocal
+    DevArray<float> rows_f_;       // [F][row] scaled parameters and padded thresholds
+    DevArray<uint32_t> units_;     // [chunks][codes][cap] first feature / 8 and the mask of its features
+    DevArray<int> unit_count_;     // [chunks][codes]
+    DevArray<int> reach_;          // largest magnitude of the level's candidates
+    DevArray<unsigned char> sort_temp_;
+};
+
+}  // namespace cf

@@ -1,0 +1,54 @@
+"""Pass 1 of the staged split search (csrc/stage.cu) against the fused search, whose bins come from feature_bin:
+threshold counts on either side of the padded rows, candidates in any order with extreme parameters, feature
+counts that leave partial units, ragged frames, and depths with and without a checked reciprocal."""
+import numpy as np
+import pytest
+
+import curfil_b200 as cf
+from tests import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from curfil_b200 import _build
+    _build.build()
+    c = cf.Context(0)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("T", [1, 31, 32, 33, 63, 64])
+@pytest.mark.parametrize("F,w,h", [(1, 33, 27), (77, 97, 71), (264, 128, 96)])
+def test_bins_equal_the_fused_search(ctx, T, F, w, h):
+    n, C = 4, 17
+    rgb, depth, labels = H.frames(seed=T + F, n=n, w=w, h=h, cells=9, classes=C)
+    ds = cf.Dataset.from_raw(ctx, rgb, depth)
+    rng = np.random.default_rng(1000 * T + F)
+    sizes = [1, 65, 700, 31, 64, 1500, 2]
+    offsets = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    s = H.random_samples(rng, n, w, h, C, int(offsets[-1]), depth=depth, flips=True)
+    # depths in whole millimetres without a checked reciprocal, invalid ones, and far outside the usual range
+    odd = np.array([0.3, 0.36, 0.6, 0.72, 1.2, 2.4, 0.0, -1.0, np.nan, np.inf, 1e-4, 1e-3, 1e6, 3e7, 1.2345678],
+                   np.float32)
+    pick = rng.random(len(s)) < 0.3
+    s["depth"][pick] = rng.choice(odd, int(pick.sum()))
+    fe = H.random_features(rng, F)                     # depth and colour candidates in random order
+    fe[1:5, : F // 4] = rng.choice(np.array([-128, -127, 0, 127], np.int8), (4, F // 4))
+    fe[5:9, : F // 5] = rng.choice(np.array([-5, 0, 1, 127], np.int8), (4, F // 5))
+    r = cf.feature_responses(ds, s, fe)
+    th = np.empty((T, F), np.float32)
+    for t in range(T):
+        th[t] = np.nan_to_num(r[np.arange(F), rng.integers(0, len(s), F)], nan=0.0)
+    out = {}
+    try:
+        for stage in (0, 2):
+            ctx.set_tuning(stage_bins=stage, stage_max_mb=1)
+            out[stage] = cf.level_left_counts(ds, offsets, s, C, fe, th)
+    finally:
+        ctx.set_tuning()
+        ds.close()
+    np.testing.assert_array_equal(out[2][1], out[0][1])
+    for k in ("score", "feature", "threshold_index", "threshold"):
+        np.testing.assert_array_equal(out[2][0][k], out[0][0][k], err_msg=k)
