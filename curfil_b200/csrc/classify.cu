@@ -2,10 +2,10 @@
 //
 // Replaces classifyKernel + normalizeProbabilitiesKernel + maxProbabilitiesKernel
 // (random_tree_image_gpu.cu:1237-1453), launched once per tree per image in the reference, by one
-// launch over all trees and all frames of a batch (frames may differ in size). One thread per
-// pixel: its depth comes from the integral image as on the reference's CPU path
-// (random_tree_image.h:140-165); each tree is walked with the exact double feature response,
-// NaN going right; the leaf histograms are summed in registers, normalised by their double sum
+// launch over all trees and all frames of a batch (frames may differ in size). One, two or four
+// threads per pixel: its depth comes from the integral image as on the reference's CPU path
+// (random_tree_image.h:140-165); each tree is walked with the decisions of the exact double feature
+// response, NaN going right; the leaf histograms are summed in registers, normalised by their double sum
 // and arg-maxed with the lowest label winning ties (random_forest_image.cpp:307-345). The top
 // levels of every tree are staged in shared memory, the rest is read through L1/L2.
 #include <algorithm>
@@ -13,7 +13,7 @@
 #include <cstring>
 #include <memory>
 
-#include "eval_fast.cuh"
+#include "box_fast.cuh"
 #include "features.h"
 #include "forest.h"
 
@@ -21,41 +21,87 @@ namespace cf {
 
 namespace {
 
-constexpr int kClassifyThreads = 256;
-constexpr int kSmemNodesBudget = 2048;  // 32 KB of cached nodes per CTA
+constexpr int kSmemNodesBudget = 256;   // 4 KB of cached nodes per CTA (2048: 3 % slower, less L1 for the corners)
 constexpr int kTreeChunk = 32;          // trees walked before their leaves are summed
-constexpr int kTileW = 32, kTileH = 8;  // pixels of one classify CTA (8 warps of 8x4)
+constexpr int kDepths = 65536;          // table of checked reciprocals, by depth in mm
+constexpr int kTileW = 16, kTileH = 16;   // pixels of a classify tile
 
-__device__ __forceinline__ float pixel_depth(const int2* D, int W, int x, int y) {
+// Depth of a pixel in mm from the integral image (<= 0: invalid).
+__device__ __forceinline__ int pixel_mm(const int2* D, int W, int x, int y) {
     const int2 c = __ldg(D + static_cast<long long>(y) * W + x);
     const int2 a = y > 0 ? __ldg(D + static_cast<long long>(y - 1) * W + x) : make_int2(0, 0);
     const int2 l = x > 0 ? __ldg(D + static_cast<long long>(y) * W + x - 1) : make_int2(0, 0);
     const int2 al = (x > 0 && y > 0) ? __ldg(D + static_cast<long long>(y - 1) * W + x - 1) : make_int2(0, 0);
     const int valid = c.y - (l.y + a.y - al.y);
-    if (valid != 1) return 0.0f;
-    const int mm = static_cast<int>(static_cast<uint32_t>(c.x) -
-                                    (static_cast<uint32_t>(l.x) + static_cast<uint32_t>(a.x) - static_cast<uint32_t>(al.x)));
-    if (mm <= 0) return 0.0f;
-    return __fdiv_rn(static_cast<float>(mm), 1000.0f);
+    if (valid != 1) return 0;
+    return static_cast<int>(static_cast<uint32_t>(c.x) -
+                            (static_cast<uint32_t>(l.x) + static_cast<uint32_t>(a.x) - static_cast<uint32_t>(al.x)));
 }
 
-// A CTA covers 32x8 pixels, each warp an 8x4 tile, so the lanes of a warp are close in both
-// directions and mostly walk the same nodes. Each lane moves on to its next tree as soon as it
-// reaches a leaf (lanes do not wait at tree boundaries for the deepest path of the warp) and only
-// records the leaf ([tree][threads] after the node cache); the histograms are summed afterwards,
-// all lanes together, in tree order.
-template <int CMAX>
-__global__ void __launch_bounds__(kClassifyThreads, CMAX <= 64 ? 4 : 1)
+__device__ __forceinline__ float depth_of(int mm) { return mm > 0 ? __fdiv_rn(static_cast<float>(mm), 1000.0f) : 0.0f; }
+
+__device__ __forceinline__ float pixel_depth(const int2* D, int W, int x, int y) { return depth_of(pixel_mm(D, W, x, y)); }
+
+// The checked reciprocal of every depth of up to 65535 mm (0: none), for node parameters of up to 128.
+__global__ void reciprocals_kernel(float* __restrict__ inv) {
+    const int mm = blockIdx.x * blockDim.x + threadIdx.x;
+    if (mm < kDepths) inv[mm] = mm > 0 ? checked_reciprocal(depth_of(mm), 128) : 0.0f;
+}
+
+// The side of one node for a pixel without a checked reciprocal (feature_bin).
+__device__ __noinline__ int general_side(const FrameDesc* fr, int x, int y, float depth, const PackedNode nd) {
+    EvalPixel px;
+    px.color = fr->color;
+    px.depth = fr->depth;
+    px.x = x;
+    px.y = y;
+    px.d = depth;
+    px.inv_d = depth > 0.0f ? __frcp_rn(depth) : 0.0f;
+    const EvalFeat ef = eval_feat_of(nd.o1x, nd.o1y, nd.o2x, nd.o2y, nd.r1x, nd.r1y, nd.r2x, nd.r2y, (nd.meta >> 26) & 1u,
+                                     (nd.meta >> 27) & 3u, (nd.meta >> 29) & 3u);
+    return feature_bin(px, fr->width, fr->height, ef, false, ThresholdSide{nd.threshold});
+}
+
+// Two of four signed bytes (each plus 128) as floats: 2^23 + 128 + v in the bits, less 2^23 + 128.
+__device__ __forceinline__ u64 byte_pair(uint32_t biased, uint32_t at) {
+    const float a = __uint_as_float(__byte_perm(biased, 0x4B000000u, 0x7650u + at));
+    const float b = __uint_as_float(__byte_perm(biased, 0x4B000000u, 0x7651u + at));
+    return sub2(pack_f2(a, b), pack_f2(8388736.0f, 8388736.0f));
+}
+
+// 2^23 with the signs of two floats
+__device__ __forceinline__ u64 sign_pair(u64 v) { return (v & 0x8000000080000000ull) | 0x4B0000004B000000ull; }
+
+// A CTA takes half or a quarter of a 16 x 16 tile; warps take 8 x 4 pixels, so the lanes of a warp are close in
+// both directions and mostly walk the same nodes. kSplit threads share a
+// pixel: each walks every kSplit-th tree (moving on to its next tree as soon as it reaches a leaf, so lanes
+// do not wait at tree boundaries for the deepest path of the warp) and records only the leaves; then each
+// sums its share of the classes over all leaves, in tree order, the double sum is passed from share to
+// share in class order, and each normalises its own classes. The results are those of one thread per pixel.
+// With two threads per pixel half as many pixels are in flight per SM and their corners stay in L1 more often
+// (sector hit rate 47 -> 71 %), and 20 class sums instead of 40 fit in the registers beside the walk. The
+// kernel is bound by instruction issue (73 %) and the L1 tag pipe (73 %): 41 000 warp instructions for 32
+// pixels of 10 trees, 65 700 before the walk used box_fast.cuh; 64 frames 640x480, 40 classes: 39.0 -> 28.4 ms.
+template <int CMAX, int kPixels, int kSplit>
+__global__ void __launch_bounds__(kPixels * kSplit, CMAX / kSplit <= 32 ? 1024 / (kPixels * kSplit) : 1)
 classify_kernel(const PackedNode* __restrict__ nodes, const int* __restrict__ tree_base, int num_trees, int cache,
-                const float* __restrict__ leaves, int C, const FrameDesc* __restrict__ frames, int num_frames) {
+                const float* __restrict__ leaves, int leaf_stride, int C, const FrameDesc* __restrict__ frames,
+                int num_frames, const float* __restrict__ inv_mm) {
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ double s_sum[kPixels];
+    __shared__ float s_best[kPixels * kSplit];
+    __shared__ uint8_t s_label[kPixels * kSplit];
+    constexpr int kParts = kTileW * kTileH / kPixels;   // CTAs of a tile
+    constexpr int kQuads = (CMAX / 4 + kSplit - 1) / kSplit;
     PackedNode* s_nodes = reinterpret_cast<PackedNode*>(smem);
-    uint32_t* my_leaf = reinterpret_cast<uint32_t*>(smem + sizeof(PackedNode) * num_trees * cache) + threadIdx.x;
+    const int pixel = threadIdx.x % kPixels, share = threadIdx.x / kPixels;
+    uint32_t* leaf = reinterpret_cast<uint32_t*>(smem + sizeof(PackedNode) * num_trees * cache) + pixel;   // [tree][kPixels]
+    const int tile = static_cast<int>(blockIdx.x) / kParts;
     // which frame does this CTA serve
     int lo = 0, hi = num_frames - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (frames[mid].first_block <= static_cast<int>(blockIdx.x)) lo = mid; else hi = mid - 1;
+        if (frames[mid].first_block <= tile) lo = mid; else hi = mid - 1;
     }
     const FrameDesc fr = frames[lo];
     // stage the top `cache` nodes of every tree
@@ -66,80 +112,150 @@ classify_kernel(const PackedNode* __restrict__ nodes, const int* __restrict__ tr
     }
     __syncthreads();
     const long long plane = static_cast<long long>(fr.width) * fr.height;
-    const int b = static_cast<int>(blockIdx.x) - fr.first_block;
+    const int b = tile - fr.first_block;
     const int bw = (fr.width + kTileW - 1) / kTileW;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int x = (b % bw) * kTileW + (warp & 3) * 8 + (lane & 7);
-    const int y = (b / bw) * kTileH + (warp >> 2) * 4 + (lane >> 3);
-    if (x >= fr.width || y >= fr.height) return;
+    const int lane = threadIdx.x & 31;
+    const int wt = pixel / 32 + static_cast<int>(blockIdx.x) % kParts * (kPixels / 32);   // 8 x 4 block of the tile
+    const int x = (b % bw) * kTileW + (wt & 1) * 8 + (lane & 7);
+    const int y = (b / bw) * kTileH + (wt >> 1) * 4 + (lane >> 3);
+    const bool inside = x < fr.width && y < fr.height;
     const long long p = static_cast<long long>(y) * fr.width + x;
-    const float depth = pixel_depth(fr.depth, fr.width, x, y);
-    EvalPixel px;
-    px.color = fr.color;
-    px.depth = fr.depth;
-    px.x = x;
-    px.y = y;
-    px.d = depth;
-    px.inv_d = depth > 0.0f ? __frcp_rn(depth) : 0.0f;
+    const int mm = inside ? pixel_mm(fr.depth, fr.width, x, y) : 0;
+    BoxLane px;
+    // an invalid depth goes right at every node: the pixel is put outside the frame
+    const float inv_d = mm > 0 && mm < kDepths && plane <= kMaxBoxPlane ? __ldg(inv_mm + mm) : 0.0f;
+    const bool general = mm > 0 && inv_d == 0.0f;
+    px.pos = pack_f2(mm > 0 ? static_cast<float>(x) : -1e6f, static_cast<float>(y));
+    px.inv = pack_f2(inv_d, inv_d);
+    px.side = pack_f2(1.0f, 1.0f);
+    FrameView view;
+    view.xmax = static_cast<float>(fr.width - 1);
+    view.ymax = static_cast<float>(fr.height - 1);
 
-    float acc[CMAX];
+    const int q0 = min(share * kQuads, (C + 3) / 4), q1 = min(q0 + kQuads, (C + 3) / 4);
+    float acc[4 * kQuads];
     for (int t0 = 0; t0 < num_trees; t0 += kTreeChunk) {
         const int t1 = min(num_trees, t0 + kTreeChunk);
-        int t = t0, idx = 0;
-        int base = tree_base[t];
-        int cached = min(cache, tree_base[t + 1] - base);
-        while (t < t1) {
-            const PackedNode nd = idx < cached ? s_nodes[t * cache + idx] : nodes[base + idx];
-            const uint32_t meta = nd.meta;
-            if (meta & 0x80000000u) {
-                my_leaf[(t - t0) * kClassifyThreads] = meta & 0x7FFFFFFFu;
-                if (++t < t1) {
-                    base = tree_base[t];
-                    cached = min(cache, tree_base[t + 1] - base);
-                }
-                idx = 0;
-                continue;
+        if (inside) {
+            int t = t0 + share, idx = 0, base = 0, cached = 0;
+            if (t < t1) {
+                base = tree_base[t];
+                cached = min(cache, tree_base[t + 1] - base);
             }
-            // !(r <= threshold) for the exact double response (NaN right), decided on the fast
-            // path unless the threshold lies within its error bound
-            const EvalFeat ef = eval_feat_of(nd.o1x, nd.o1y, nd.o2x, nd.o2y, nd.r1x, nd.r1y, nd.r2x, nd.r2y,
-                                             (meta >> 26) & 1u, (meta >> 27) & 3u, (meta >> 29) & 3u);
-            idx = static_cast<int>(meta & 0x03FFFFFFu) +
-                  feature_bin(px, fr.width, fr.height, ef, false, ThresholdSide{nd.threshold});
+            while (t < t1) {
+                const PackedNode nd = idx < cached ? s_nodes[t * cache + idx] : nodes[base + idx];
+                const uint32_t meta = nd.meta;
+                if (meta & 0x80000000u) {
+                    leaf[(t - t0) * kPixels] = meta & 0x7FFFFFFFu;
+                    t += kSplit;
+                    if (t < t1) {
+                        base = tree_base[t];
+                        cached = min(cache, tree_base[t + 1] - base);
+                    }
+                    idx = 0;
+                    continue;
+                }
+                // !(r <= threshold) for the exact double response (NaN right), decided from bounds unless the
+                // threshold lies between them
+                int side;
+                if (general) {
+                    side = general_side(frames + lo, x, y, depth_of(mm), nd);
+                } else {
+                    const uint32_t* par = reinterpret_cast<const uint32_t*>(&nd);
+                    const uint32_t off = par[0] ^ 0x80808080u, reg = par[1] ^ 0x80808080u;
+                    const u64 o1 = byte_pair(off, 0), o2 = byte_pair(off, 2);
+                    const bool color = meta >> 26 & 1u;
+                    view.size = __int_as_float(color ? 4 : 8);
+                    view.pitch = __int_as_float(color ? 4 * fr.width : 8 * fr.width);
+                    view.base1 = __int_as_float(color ? static_cast<int>(meta >> 27 & 3u) * static_cast<int>(plane) * 4 : 0);
+                    view.base2 = __int_as_float(color ? static_cast<int>(meta >> 29 & 3u) * static_cast<int>(plane) * 4 : 0);
+                    const Corners k =
+                        corners(px, o1, o2, byte_pair(reg, 0), byte_pair(reg, 2), sign_pair(o1), sign_pair(o2), view);
+                    side = 1;
+                    if (color) {
+                        const double r = color_response(k, reinterpret_cast<const unsigned char*>(fr.color));
+                        if (k.in && r <= static_cast<double>(nd.threshold)) side = 0;
+                    } else {
+                        const DepthBoxes box = depth_boxes(k, reinterpret_cast<const unsigned char*>(fr.depth));
+                        if (k.in && box.n1 != 0 && box.n2 != 0) {
+                            const DepthBounds d = depth_bounds(box);
+                            if (d.plain && d.hi < nd.threshold) side = 0;
+                            else if (!(d.plain && d.lo > nd.threshold))
+                                side = exact_depth_response(box.s1, box.n1, box.s2, box.n2) <= static_cast<double>(nd.threshold) ? 0 : 1;
+                        }
+                    }
+                }
+                idx = static_cast<int>(meta & 0x03FFFFFFu) + side;
+            }
         }
+        if (kSplit > 1) __syncthreads();
         // the leaves' normalised histograms, summed in tree order as the reference sums them
-        for (int tt = t0; tt < t1; tt++) {
-            const float* row = leaves + static_cast<long long>(my_leaf[(tt - t0) * kClassifyThreads]) * C;
+        for (int tt = t0; inside && tt < t1; tt++) {
+            // rows padded to whole quads: a 16-byte load takes the same tag lookups as a 4-byte one
+            const float4* row =
+                reinterpret_cast<const float4*>(leaves + static_cast<long long>(leaf[(tt - t0) * kPixels]) * leaf_stride) + q0;
 #pragma unroll
-            for (int c = 0; c < CMAX; c++)
-                if (c < C) acc[c] = __fadd_rn(tt == 0 ? 0.0f : acc[c], __ldg(row + c));
+            for (int q = 0; q < kQuads; q++)
+                if (q0 + q < q1) {
+                    const float4 v = __ldg(row + q);
+                    acc[4 * q] = __fadd_rn(tt == 0 ? 0.0f : acc[4 * q], v.x);
+                    acc[4 * q + 1] = __fadd_rn(tt == 0 ? 0.0f : acc[4 * q + 1], v.y);
+                    acc[4 * q + 2] = __fadd_rn(tt == 0 ? 0.0f : acc[4 * q + 2], v.z);
+                    acc[4 * q + 3] = __fadd_rn(tt == 0 ? 0.0f : acc[4 * q + 3], v.w);
+                }
         }
+        if (kSplit > 1 && t1 < num_trees) __syncthreads();   // the leaves are read before the next trees' come
     }
-    auto acc_of = [&](int c) { return acc[c]; };
+    // the sum over the classes in class order, share by share
     double sum = 0.0;
 #pragma unroll
-    for (int c = 0; c < CMAX; c++)
-        if (c < C) sum = __dadd_rn(sum, static_cast<double>(acc_of(c)));
+    for (int g = 0; g < kSplit; g++) {
+        if (g == share) {
+            if (g > 0) sum = s_sum[pixel];
+#pragma unroll
+            for (int c = 0; c < 4 * kQuads; c++)
+                if (inside && 4 * q0 + c < C && c < 4 * (q1 - q0)) sum = __dadd_rn(sum, static_cast<double>(acc[c]));
+            if (kSplit > 1) s_sum[pixel] = sum;
+        }
+        if (kSplit > 1) __syncthreads();
+    }
+    if (kSplit > 1) sum = s_sum[pixel];
     // RN(acc / sum) from the correctly rounded reciprocal with one correction step (Markstein,
     // IBM J. Res. Dev. 34(1), 1990): q = RN(a y), r = a - q sum exactly by FMA, RN(q + r y)
     const double inv = __drcp_rn(sum);
     float best = -1.0f;
     int label = 0;
 #pragma unroll
-    for (int c = 0; c < CMAX; c++) {
-        if (c < C) {
-            const double a = static_cast<double>(acc_of(c));
+    for (int c = 0; c < 4 * kQuads; c++) {
+        if (inside && 4 * q0 + c < C && c < 4 * (q1 - q0)) {
+            const double a = static_cast<double>(acc[c]);
             const double q = __dmul_rn(a, inv);
             const double q1 = __fma_rn(__fma_rn(-q, sum, a), inv, q);
             const float v = __double2float_rn(q1);
-            if (fr.probs) fr.probs[c * plane + p] = v;
+            if (fr.probs) fr.probs[(4 * q0 + c) * plane + p] = v;
             if (v > best) {
                 best = v;
-                label = c;
+                label = 4 * q0 + c;
             }
         }
     }
-    if (fr.labels) fr.labels[p] = static_cast<uint8_t>(label);
+    if (!fr.labels) return;   // the same for the whole CTA
+    if (kSplit == 1) {
+        if (inside) fr.labels[p] = static_cast<uint8_t>(label);
+        return;
+    }
+    // the lowest label of the best: shares in class order, a later one only where it is better
+    s_best[threadIdx.x] = best;
+    s_label[threadIdx.x] = static_cast<uint8_t>(label);
+    __syncthreads();
+    if (share == 0 && inside) {
+        for (int g = 1; g < kSplit; g++)
+            if (s_best[g * kPixels + pixel] > best) {
+                best = s_best[g * kPixels + pixel];
+                label = s_label[g * kPixels + pixel];
+            }
+        fr.labels[p] = static_cast<uint8_t>(label);
+    }
 }
 
 // ---- the plain per-image launch form (classifyImage, random_tree_image_gpu.cu:1414-1453): per image
@@ -147,7 +263,7 @@ classify_kernel(const PackedNode* __restrict__ nodes, const int* __restrict__ tr
 // histogram into probabilities [C][H][W] in global memory, then a normalisation launch and an
 // argmax launch, each followed by a stream synchronisation as the reference's mutex-guarded loop.
 __global__ void plain_classify_tree_kernel(const PackedNode* __restrict__ nodes, int base,
-                                           const float* __restrict__ leaves, int C, FrameDesc fr) {
+                                           const float* __restrict__ leaves, int leaf_stride, int C, FrameDesc fr) {
     const long long plane = static_cast<long long>(fr.width) * fr.height;
     const long long p = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (p >= plane) return;
@@ -183,7 +299,7 @@ __global__ void plain_classify_tree_kernel(const PackedNode* __restrict__ nodes,
         const double r = feature_response(ds, 0, x, y, depth, fp, false);
         idx = static_cast<int>(meta & 0x03FFFFFFu) + ((r <= static_cast<double>(nd.threshold)) ? 0 : 1);
     }
-    const float* row = leaves + static_cast<long long>(meta & 0x7FFFFFFFu) * C;
+    const float* row = leaves + static_cast<long long>(meta & 0x7FFFFFFFu) * leaf_stride;
     for (int c = 0; c < C; c++) fr.probs[c * plane + p] = __fadd_rn(fr.probs[c * plane + p], __ldg(row + c));
 }
 
@@ -211,19 +327,40 @@ __global__ void plain_argmax_kernel(const float* __restrict__ probs, int C, long
     labels[p] = static_cast<uint8_t>(label);
 }
 
-template <int CMAX>
+template <int CMAX, int kPixels, int kSplit>
 void launch_classify(cf_context* ctx, cudaStream_t stream, const cf_forest* f, const FrameDesc* frames, int num_frames,
                      int blocks) {
     const size_t smem = sizeof(PackedNode) * f->num_trees * f->cache_per_tree +
-                        sizeof(uint32_t) * std::min(f->num_trees, kTreeChunk) * kClassifyThreads;
-    auto kernel = classify_kernel<CMAX>;
+                        sizeof(uint32_t) * std::min(f->num_trees, kTreeChunk) * kPixels;
+    auto kernel = classify_kernel<CMAX, kPixels, kSplit>;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CF_CUDA_CHECK(cudaStreamIsCapturing(stream, &cs));
     if (cs == cudaStreamCaptureStatusNone)   // set before capture (an uncaptured pass runs first)
         CF_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            static_cast<int>(std::max<size_t>(smem, 1))));
-    launch_on(ctx, stream, "classify", dim3(blocks), dim3(kClassifyThreads), smem, kernel, f->nodes.get(),
-              f->d_tree_base.get(), f->num_trees, f->cache_per_tree, f->leaves.get(), f->C, frames, num_frames);
+    launch_on(ctx, stream, "classify", dim3(blocks * (kTileW * kTileH / kPixels)), dim3(kPixels * kSplit), smem, kernel,
+              f->nodes.get(), f->d_tree_base.get(), f->num_trees, f->cache_per_tree, f->leaves.get(), f->leaf_stride, f->C,
+              frames, num_frames, f->inv_mm.get());
+}
+
+// Two threads per pixel and half tiles (10 trees, 40 classes, 64 frames 640x480: 28.4 ms; one thread 33.3 ms,
+// four 30.0 ms), except one thread for one or three trees, which do not halve, where its class sums fit the
+// registers (3 trees, 13 classes, 4 frames: 479 against 521 us); and four threads and quarter tiles for
+// launches of few tiles, which the longest walk bounds (160x120, 3 trees: 38 against 56 us).
+template <int CMAX>
+void launch_classify(cf_context* ctx, cudaStream_t stream, const cf_forest* f, const FrameDesc* frames, int num_frames,
+                     int blocks) {
+    if (blocks < 4 * ctx->num_sms) {
+        launch_classify<CMAX, 64, 4>(ctx, stream, f, frames, num_frames, blocks);
+        return;
+    }
+    if constexpr (CMAX <= 32) {
+        if (f->num_trees == 1 || f->num_trees == 3) {
+            launch_classify<CMAX, 128, 1>(ctx, stream, f, frames, num_frames, blocks);
+            return;
+        }
+    }
+    launch_classify<CMAX, 128, 2>(ctx, stream, f, frames, num_frames, blocks);
 }
 
 }  // namespace
@@ -308,6 +445,8 @@ cf_status cf_forest_create(cf_context* ctx, int num_trees, cf_tree* const* trees
         std::vector<float> leaves;
         std::vector<int> base(num_trees + 1, 0);
         std::vector<double> norm(C);
+        const int stride = (C + 3) & ~3;
+        f->leaf_stride = stride;
         for (int t = 0; t < num_trees; t++) {
             const cf_tree* tr = trees[t];
             base[t] = static_cast<int>(packed.size());
@@ -327,9 +466,9 @@ cf_status cf_forest_create(cf_context* ctx, int num_trees, cf_tree* const* trees
                 if (tr->left[i] < 0) {
                     normalize_histogram(C, &tr->hist[static_cast<size_t>(i) * C], pr, histogram_bias,
                                         use_labels_prior != 0, norm.data());
-                    const int64_t row = static_cast<int64_t>(leaves.size() / C);
+                    const int64_t row = static_cast<int64_t>(leaves.size() / stride);
                     CF_REQUIRE(row < 0x7FFFFFFF, "too many leaves");
-                    for (int c = 0; c < C; c++) leaves.push_back(static_cast<float>(norm[c]));
+                    for (int c = 0; c < stride; c++) leaves.push_back(c < C ? static_cast<float>(norm[c]) : 0.0f);
                     pn.threshold = std::nanf("");
                     pn.meta = 0x80000000u | static_cast<uint32_t>(row);
                 } else {
@@ -344,7 +483,7 @@ cf_status cf_forest_create(cf_context* ctx, int num_trees, cf_tree* const* trees
         base[num_trees] = static_cast<int>(packed.size());
         f->tree_base = base;
         f->num_nodes = static_cast<int64_t>(packed.size());
-        f->num_leaves = static_cast<int64_t>(leaves.size() / C);
+        f->num_leaves = static_cast<int64_t>(leaves.size() / stride);
         f->cache_per_tree = std::max(1, kSmemNodesBudget / num_trees);
         f->nodes.reserve(packed.size());
         f->d_tree_base.reserve(base.size());
@@ -355,6 +494,8 @@ cf_status cf_forest_create(cf_context* ctx, int num_trees, cf_tree* const* trees
                                       cudaMemcpyHostToDevice, ctx->stream));
         CF_CUDA_CHECK(cudaMemcpyAsync(f->leaves.get(), leaves.data(), sizeof(float) * leaves.size(),
                                       cudaMemcpyHostToDevice, ctx->stream));
+        f->inv_mm.reserve(kDepths);
+        launch(ctx, "reciprocals", dim3(kDepths / 256), dim3(256), 0, reciprocals_kernel, f->inv_mm.get());
         CF_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
         context_retain(ctx);
         *out = guard_f.release();
@@ -525,7 +666,7 @@ cf_status cf_predict_dataset_plain(cf_forest* forest, cf_dataset* ds, int first,
             CF_CUDA_CHECK(cudaMemsetAsync(fr.probs, 0, sizeof(float) * C * plane, st));
             for (int t = 0; t < forest->num_trees; t++) {
                 launch(ctx, "plain_classify", dim3(blocks), dim3(256), 0, plain_classify_tree_kernel, forest->nodes.get(),
-                       forest->tree_base[t], forest->leaves.get(), C, fr);
+                       forest->tree_base[t], forest->leaves.get(), forest->leaf_stride, C, fr);
                 CF_CUDA_CHECK(cudaStreamSynchronize(st));
             }
             launch(ctx, "plain_normalize", dim3(blocks), dim3(256), 0, plain_normalize_kernel, fr.probs, C, plane);
@@ -574,7 +715,7 @@ cf_status cf_predict_host_plain(cf_forest* forest, int count, int width, int hei
             CF_CUDA_CHECK(cudaMemsetAsync(fr.probs, 0, sizeof(float) * C * plane, st));
             for (int t = 0; t < forest->num_trees; t++) {
                 launch(ctx, "plain_classify", dim3(blocks), dim3(256), 0, plain_classify_tree_kernel, forest->nodes.get(),
-                       forest->tree_base[t], forest->leaves.get(), C, fr);
+                       forest->tree_base[t], forest->leaves.get(), forest->leaf_stride, C, fr);
                 CF_CUDA_CHECK(cudaStreamSynchronize(st));
             }
             const long long pl = static_cast<long long>(plane);

@@ -48,7 +48,9 @@ struct cf_forest {
     std::vector<int> tree_base;      // first node of each tree in `nodes`
     cf::DevArray<cf::PackedNode> nodes;
     cf::DevArray<int> d_tree_base;
-    cf::DevArray<float> leaves;      // [L][C] normalised histograms (float, as convertTree stores them)
+    int leaf_stride = 0;             // floats of a leaf row: C rounded up to a multiple of 4, the rest 0
+    cf::DevArray<float> leaves;      // [L][leaf_stride] normalised histograms (float, as convertTree stores them)
+    cf::DevArray<float> inv_mm;      // [65536] checked reciprocal of each depth in mm
     int64_t num_leaves = 0;
     // scratch of cf_predict_host
     cf::DevArray<uint8_t> raw_rgb;

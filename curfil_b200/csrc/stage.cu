@@ -23,14 +23,12 @@
 
 #include <cub/device/device_radix_sort.cuh>
 
-#include "eval_fast.cuh"
+#include "box_fast.cuh"
 #include "stage.h"
 
 namespace cf {
 
 namespace {
-
-using u64 = unsigned long long;
 
 constexpr int kThreads = 512;         // 16 warps: kRows / 32 groups of lanes x 8 unit columns
 constexpr int kCtasPerSm = 2;         // 64 registers; the shared memory left over is L1
@@ -119,21 +117,6 @@ stage_units_kernel(int F, int chunk, int cap, const FeatParams* __restrict__ pac
     if (threadIdx.x < kStageCodes) unit_count[blockIdx.x * kStageCodes + threadIdx.x] = s_n[threadIdx.x];
 }
 
-// A float i with floor(v i) = trunc(RN(v / d)) for v = 1 .. most (RN(1 / d) or the next float), or 0.
-__device__ __forceinline__ float checked_reciprocal(float d, int most) {
-    float inv = __frcp_rn(d);
-    for (int k = 0; k < 2; k++) {
-        bool same = true;
-        for (int v = 1; v <= most && same; v++) {
-            const float f = __uint2float_rn(v);
-            same = __fmaf_rz(f, inv, 8388608.0f) == __fadd_rz(__fdiv_rn(f, d), 8388608.0f);
-        }
-        if (same) return inv;
-        inv = __uint_as_float(__float_as_uint(inv) + 1u);
-    }
-    return 0.0f;
-}
-
 // Rows of the table: row_base[n] + k is sample k of node n. Pass 1 takes them frame by frame and within a
 // frame in Morton (Z) order of (y, x), so that the rows a CTA takes lie in a compact patch; rows without a
 // checked reciprocal come last, in the same order.
@@ -210,51 +193,6 @@ __device__ __forceinline__ uint8_t* bin_place(const StageArgs& a, int g, long lo
     return a.out + (((g >> 5) * a.rows + row) << 5) + (g & 31);
 }
 
-// ---- two floats per instruction -----------------------------------------------------------------
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ u64 fma2_rz(u64 a, u64 b, u64 c) {
-    u64 r;
-    asm("fma.rz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ u64 add2(u64 a, u64 b) {
-    u64 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 sub2(u64 a, u64 b) {
-    u64 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(u64 v) {
-    float2 r;
-    unpack_f2(v, r.x, r.y);
-    return r;
-}
-
-// What a lane holds of its sample, and of the frame for the features at hand.
-struct Lane {
-    u64 pos;        // (x, y)
-    u64 inv;        // the sample's checked reciprocal, twice
-    u64 side;       // (1 or -1 for a flipped response, 1)
-};
-
-// Bytes of an element and of a row and the first bytes of the planes of box 1 and box 2, as multiples of the
-// smallest denormal: such a float's bits are the integer, up to 2^24, so offsets need no conversion.
-struct FrameView {
-    float xmax, ymax, size, pitch, base1, base2;
-};
-
-// trunc(RN(v / d)) of two parameters; big = 2^23 with each value's sign
-__device__ __forceinline__ u64 scale2(u64 v, const Lane& l, u64 big) {
-    return sub2(fma2_rz(v, l.inv, big), big);
-}
-
 // Thresholds below v of a padded row (32 entries serve T <= 31, 36 T = 32, 64 T <= 63): halving, on a byte
 // offset so that a step is a read, a compare and an addition.
 template <int kRow>
@@ -274,88 +212,25 @@ __device__ __forceinline__ int row_below(const float* t, float v) {
     return kEntries == 36 ? k + (t[31] < v ? 1 : 0) : k;
 }
 
-// The two boxes of one feature: byte offsets of their corners in the sample's frame, and whether both
-// lie inside it.
-struct Corners {
-    int ul1, ur1, ll1, lr1, ul2, ur2, ll2, lr2;
-    bool in;
-};
-
-__device__ __forceinline__ Corners corners(const Lane& l, const float* row, const FrameView& p) {
+__device__ __forceinline__ Corners row_corners(const BoxLane& l, const float* row, const FrameView& p) {
     const ulonglong2 o = *reinterpret_cast<const ulonglong2*>(row);          // o1, o2
     const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(row + 4);      // r1, r2
     const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(row + 8);      // 2^23 with the offsets' signs
-    const u64 big = pack_f2(8388608.0f, 8388608.0f);
-    const u64 c1 = fma2(scale2(o.x, l, b.x), l.side, l.pos);
-    const u64 c2 = fma2(scale2(o.y, l, b.y), l.side, l.pos);
-    const float2 g1 = unpack2(scale2(g.x, l, big)), g2 = unpack2(scale2(g.y, l, big));
-    const float w1 = fmaxf(g1.x, 1.0f), h1 = fmaxf(g1.y, 1.0f), w2 = fmaxf(g2.x, 1.0f), h2 = fmaxf(g2.y, 1.0f);
-    const u64 s1 = pack_f2(w1, h1), s2 = pack_f2(w2, h2);
-    const float2 lo1 = unpack2(sub2(c1, s1)), hi1 = unpack2(add2(c1, s1));
-    const float2 lo2 = unpack2(sub2(c2, s2)), hi2 = unpack2(add2(c2, s2));
-    Corners k;
-    k.in = fminf(fminf(lo1.x, lo1.y), fminf(lo2.x, lo2.y)) >= 0.0f && fmaxf(hi1.x, hi2.x) <= p.xmax &&
-           fmaxf(hi1.y, hi2.y) <= p.ymax;
-    const float l1 = fmaf(lo1.x, p.size, p.base1), r1 = fmaf(hi1.x, p.size, p.base1);
-    const float l2 = fmaf(lo2.x, p.size, p.base2), r2 = fmaf(hi2.x, p.size, p.base2);
-    k.ul1 = __float_as_int(fmaf(lo1.y, p.pitch, l1));
-    k.ur1 = __float_as_int(fmaf(lo1.y, p.pitch, r1));
-    k.ll1 = __float_as_int(fmaf(hi1.y, p.pitch, l1));
-    k.lr1 = __float_as_int(fmaf(hi1.y, p.pitch, r1));
-    k.ul2 = __float_as_int(fmaf(lo2.y, p.pitch, l2));
-    k.ur2 = __float_as_int(fmaf(lo2.y, p.pitch, r2));
-    k.ll2 = __float_as_int(fmaf(hi2.y, p.pitch, l2));
-    k.lr2 = __float_as_int(fmaf(hi2.y, p.pitch, r2));
-    return k;
+    return corners(l, o.x, o.y, g.x, g.y, b.x, b.y, p);
 }
 
-template <typename V>
-__device__ __forceinline__ V frame_at(const unsigned char* frame, int offset) {
-    return __ldg(reinterpret_cast<const V*>(frame + offset));
-}
-
-// The box sums and counts of a depth feature, and whether its bin still has to be found from them (a threshold
-// lies within the error bound, or a count is outside [1, 2^23)).
-struct DepthBoxes {
-    int s1, n1, s2, n2;
-    bool open;
-};
-
+// Bin of a depth feature; `open` where it still has to be found from the boxes (a threshold lies between the
+// bounds, or a count is no plain one).
 template <int kRow>
-__device__ __forceinline__ int depth_bin(const Lane& l, const float* row, const unsigned char* frame,
-                                                const FrameView& p, int T, DepthBoxes& box) {
-    const Corners k = corners(l, row, p);
-    int2 ul1 = make_int2(0, 0), ur1 = ul1, ll1 = ul1, lr1 = ul1, ul2 = ul1, ur2 = ul1, ll2 = ul1, lr2 = ul1;
-    if (k.in) {
-        ul1 = frame_at<int2>(frame, k.ul1), ur1 = frame_at<int2>(frame, k.ur1);
-        ll1 = frame_at<int2>(frame, k.ll1), lr1 = frame_at<int2>(frame, k.lr1);
-        ul2 = frame_at<int2>(frame, k.ul2), ur2 = frame_at<int2>(frame, k.ur2);
-        ll2 = frame_at<int2>(frame, k.ll2), lr2 = frame_at<int2>(frame, k.lr2);
-    }
-    auto sum = [](int lr, int ur, int ul, int ll) {
-        return static_cast<int>(static_cast<uint32_t>(lr) - static_cast<uint32_t>(ur) + static_cast<uint32_t>(ul) - static_cast<uint32_t>(ll));
-    };
-    box.s1 = sum(lr1.x, ur1.x, ul1.x, ll1.x);
-    box.n1 = sum(lr1.y, ur1.y, ul1.y, ll1.y);
-    box.s2 = sum(lr2.x, ur2.x, ul2.x, ll2.x);
-    box.n2 = sum(lr2.y, ur2.y, ul2.y, ll2.y);
-    const float n1 = __int_as_float(0x4B000000 + box.n1) - 8388608.0f;
-    const float n2 = __int_as_float(0x4B000000 + box.n2) - 8388608.0f;
-    float i1, i2;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(i1) : "f"(n1));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(i2) : "f"(n2));
-    // means in mm: the conversion is within 2^-24, the reciprocal within 2^-23, the products, the difference,
-    // 0.001f and the last rounding within 2^-24 each: the response in metres is within 4.1e-10 (a + b) of the
-    // exact one, and 5e-10 (a + b) bounds it
-    const float a = static_cast<float>(box.s1) * i1, b = static_cast<float>(box.s2) * i2;
-    const float delta = fmaf(fabsf(a) + fabsf(b), 5e-10f, 1e-30f);
-    const float r = a - b;
+__device__ __forceinline__ int depth_bin(const BoxLane& l, const float* row, const unsigned char* frame,
+                                         const FrameView& p, int T, DepthBoxes& box, bool& open) {
+    const Corners k = row_corners(l, row, p);
+    box = depth_boxes(k, frame);
+    const DepthBounds d = depth_bounds(box);
     const float* t = row + kRowParams;
-    const int bin = row_below<kRow>(t, fmaf(r, 0.001f, -delta));
-    const bool clear = t[bin] > fmaf(r, 0.001f, delta);
+    const int bin = row_below<kRow>(t, d.lo);
     const bool some = k.in && box.n1 != 0 && box.n2 != 0;
-    const bool plain = (static_cast<uint32_t>(box.n1 - 1) | static_cast<uint32_t>(box.n2 - 1)) < 0x7FFFFFu;
-    box.open = some && !(clear && plain);
+    open = some && !(t[bin] > d.hi && d.plain);
     return some ? bin : T;
 }
 
@@ -365,19 +240,10 @@ __device__ __noinline__ int open_bin(int s1, int n1, int s2, int n2, const float
 }
 
 template <int kRow>
-__device__ __forceinline__ int color_bin(const Lane& l, const float* row, const unsigned char* frame,
-                                                const FrameView& p, int T) {
-    const Corners k = corners(l, row, p);
-    float ul1 = 0, ur1 = 0, ll1 = 0, lr1 = 0, ul2 = 0, ur2 = 0, ll2 = 0, lr2 = 0;
-    if (k.in) {
-        ul1 = frame_at<float>(frame, k.ul1), ur1 = frame_at<float>(frame, k.ur1);
-        ll1 = frame_at<float>(frame, k.ll1), lr1 = frame_at<float>(frame, k.lr1);
-        ul2 = frame_at<float>(frame, k.ul2), ur2 = frame_at<float>(frame, k.ur2);
-        ll2 = frame_at<float>(frame, k.ll2), lr2 = frame_at<float>(frame, k.lr2);
-    }
-    const double A = __dadd_rn(__dsub_rn(lr1, ur1), __dsub_rn(ul1, ll1));
-    const double B = __dadd_rn(__dsub_rn(lr2, ur2), __dsub_rn(ul2, ll2));
-    const double r = __dsub_rn(A, B);   // NaN if a corner is
+__device__ __forceinline__ int color_bin(const BoxLane& l, const float* row, const unsigned char* frame,
+                                         const FrameView& p, int T) {
+    const Corners k = row_corners(l, row, p);
+    const double r = color_response(k, frame);
     const int bin = row_below<kRow>(row + kRowParams, __double2float_ru(r));
     return k.in && !isnan(r) ? bin : T;
 }
@@ -409,7 +275,7 @@ stage_gather_kernel(const __grid_constant__ StageArgs a) {
         const bool have = k < end;
         const StageSample s = a.list[have ? k : end - 1];
         const bool valid = s.inv_d > 0.0f;
-        Lane l;
+        BoxLane l;
         const float inv = valid ? s.inv_d : 1.0f;
         l.pos = pack_f2(static_cast<float>(s.x), static_cast<float>(s.y));
         l.inv = pack_f2(inv, inv);
@@ -450,10 +316,11 @@ stage_gather_kernel(const __grid_constant__ StageArgs a) {
                     view.base1 = view.base2 = 0.0f;
                     for (int i = 0; i < kStageUnit; i += 2, r += 2 * kRow) {
                         DepthBoxes x0, x1;
-                        int b0 = depth_bin<kRow>(l, r, depth, view, T, x0);
-                        int b1 = depth_bin<kRow>(l, r + kRow, depth, view, T, x1);
-                        if (x0.open) b0 = open_bin<kRow>(x0.s1, x0.n1, x0.s2, x0.n2, r + kRowParams);
-                        if (x1.open) b1 = open_bin<kRow>(x1.s1, x1.n1, x1.s2, x1.n2, r + kRow + kRowParams);
+                        bool open0, open1;
+                        int b0 = depth_bin<kRow>(l, r, depth, view, T, x0, open0);
+                        int b1 = depth_bin<kRow>(l, r + kRow, depth, view, T, x1, open1);
+                        if (open0) b0 = open_bin<kRow>(x0.s1, x0.n1, x0.s2, x0.n2, r + kRowParams);
+                        if (open1) b1 = open_bin<kRow>(x1.s1, x1.n1, x1.s2, x1.n2, r + kRow + kRowParams);
                         lo = __byte_perm(lo, hi, 0x5432);                        // (hi, lo) moves down two bytes
                         hi = __byte_perm(hi, __byte_perm(b0, b1, 0x0040), 0x5432);
                     }
@@ -583,7 +450,7 @@ void BinStager::prepare(cf_context* ctx, const DsView& ds, const Sample* samples
     cap_ = (chunk + kStageUnit - 1) / kStageUnit;
     // the padded threshold rows serve T <= 63, the float offsets frames of up to 2^24 bytes of depth integral
     // (1280x960: 9.8 MB); otherwise every row takes the general kernel
-    padded_ = lf.T <= kMaxPaddedT && ds.plane * 12 <= (1ll << 24);
+    padded_ = lf.T <= kMaxPaddedT && ds.plane <= kMaxBoxPlane;
     int frame_bits = 1;
     while ((1ll << frame_bits) < ds.n) frame_bits++;
     cudaStream_t st = ctx->stream;
