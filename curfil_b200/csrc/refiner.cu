@@ -17,6 +17,7 @@
 #include <random>
 #include <vector>
 
+#include "box_fast.cuh"
 #include "forest.h"
 
 struct cf_refiner {
@@ -40,6 +41,8 @@ namespace {
 constexpr int kTile = 64;        // samples per training tile
 constexpr int kMaxHidden = 128;
 constexpr int kMaxClasses = 64;
+constexpr int kPredictThreads = 256;
+constexpr int kChunk = 8;          // planes fetched at a time
 
 __device__ __forceinline__ float pixel_depth_m(const int2* D, int W, int x, int y) {
     const int2 c = __ldg(D + static_cast<long long>(y) * W + x);
@@ -80,6 +83,116 @@ __global__ void box_cols_kernel(const float* __restrict__ rows, float* __restric
         float s = 0.0f;
         for (int yy = y0; yy <= y1; yy++) s += rows[c * plane_px + static_cast<long long>(yy) * W + x];
         out[i] = s / static_cast<float>((y1 - y0 + 1) * (x1 - x0 + 1));
+    }
+}
+
+// Both box means of a class plane in one pass. A CTA copies a 64 x 64 tile with a margin of the larger radius
+// (zeros outside the frame) into shared memory, forms the row sums of both radii there and from them the
+// column sums. A thread takes eight consecutive outputs, each summed in ascending order from its own window
+// as box_rows_kernel and box_cols_kernel sum it (adding a margin's zero changes nothing), so the means are
+// bit-identical; a value is read once for eight outputs, and the lanes of a warp lie along the other axis, so
+// the odd row strides are free of bank conflicts. Bound by the additions (about 100 per output and radius 16).
+// 40 planes of 640x480, radii 4 and 16: 460 -> 125 us a frame (four launches before).
+constexpr int kBoxTile = 64, kBoxMaxRadius = 16, kBoxRun = 8;
+
+__host__ __device__ constexpr size_t box_smem(int r) {
+    return sizeof(float) * ((kBoxTile + 2 * r) * (kBoxTile + 2 * r + 1) + (kBoxTile + 2 * r) * (kBoxTile + 1));
+}
+
+// acc[i] = sum of v[i .. i + 2 r] in ascending order, v advancing by `stride`; two sums per addition
+__device__ __forceinline__ void run_sums(const float* v, int stride, int r, float (&acc)[kBoxRun]) {
+#pragma unroll
+    for (int i = 0; i < kBoxRun; i++) acc[i] = 0.0f;
+    const int n = 2 * r + 1;
+    if (n < kBoxRun) {
+        for (int p = 0; p < n + kBoxRun - 1; p++, v += stride) {
+            const float x = *v;
+#pragma unroll
+            for (int i = 0; i < kBoxRun; i++)
+                if (p >= i && p < i + n) acc[i] += x;
+        }
+        return;
+    }
+#pragma unroll
+    for (int p = 0; p < kBoxRun - 1; p++, v += stride) {
+        const float x = *v;
+#pragma unroll
+        for (int i = 0; i <= p; i++) acc[i] += x;
+    }
+    u64 pair[kBoxRun / 2];
+#pragma unroll
+    for (int i = 0; i < kBoxRun / 2; i++) pair[i] = pack_f2(acc[2 * i], acc[2 * i + 1]);
+#pragma unroll 4
+    for (int p = kBoxRun - 1; p < n; p++, v += stride) {
+        const u64 x = pack_f2(*v, *v);
+#pragma unroll
+        for (int i = 0; i < kBoxRun / 2; i++) pair[i] = add2(pair[i], x);
+    }
+#pragma unroll
+    for (int i = 0; i < kBoxRun / 2; i++) unpack_f2(pair[i], acc[2 * i], acc[2 * i + 1]);
+#pragma unroll
+    for (int p = 1; p < kBoxRun; p++, v += stride) {
+        const float x = *v;
+#pragma unroll
+        for (int i = p; i < kBoxRun; i++) acc[i] += x;
+    }
+}
+
+__global__ void __launch_bounds__(256)
+box_means_kernel(const float* __restrict__ in, float* __restrict__ out1, float* __restrict__ out2, int W, int H, int r1,
+                 int r2) {
+    extern __shared__ __align__(16) float sm[];
+    const int m = max(r1, r2), side = kBoxTile + 2 * m, stride = side + 1;
+    constexpr int kSumStride = kBoxTile + 1;
+    float* tile = sm;                             // [side][stride]
+    float* sums = tile + side * stride;           // [side][kSumStride] row sums of one radius
+    const long long plane = static_cast<long long>(blockIdx.z) * W * H;
+    const int x0 = blockIdx.x * kBoxTile, y0 = blockIdx.y * kBoxTile;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int y = warp; y < side; y += 8) {
+        const int gy = y0 + y - m;
+        const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(tile + y * stride));
+        for (int x = lane; x < side; x += 32) {
+            const int gx = x0 + x - m;
+            const bool ok = gx >= 0 && gx < W && gy >= 0 && gy < H;
+            const float* from = in + plane + (ok ? static_cast<long long>(gy) * W + gx : 0);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to + 4 * x), "l"(from), "r"(ok ? 4 : 0)
+                         : "memory");   // 0 bytes: the word is zeroed
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    constexpr int kRuns = kBoxTile / kBoxRun;
+    const int row_blocks = (side + 31) / 32;
+    for (int which = 0; which < 2; which++) {
+        const int r = which ? r2 : r1;
+        for (int t = warp; t < row_blocks * kRuns; t += 8) {
+            const int y = t / kRuns * 32 + lane, x = t % kRuns * kBoxRun;
+            if (y < m - r || y >= side - (m - r)) continue;
+            float acc[kBoxRun];
+            run_sums(tile + y * stride + x + m - r, 1, r, acc);
+            float* to = sums + y * kSumStride + x;
+#pragma unroll
+            for (int i = 0; i < kBoxRun; i++) to[i] = acc[i];
+        }
+        __syncthreads();
+        for (int t = warp; t < 2 * kRuns; t += 8) {
+            const int x = (t & 1) * 32 + lane, y = (t >> 1) * kBoxRun;
+            const int gx = x0 + x;
+            if (gx >= W) continue;
+            float acc[kBoxRun];
+            run_sums(sums + (y + m - r) * kSumStride + x, kSumStride, r, acc);
+            float* out = (which ? out2 : out1) + plane + gx;
+            const int cols = min(W - 1, gx + r) - max(0, gx - r) + 1;
+#pragma unroll
+            for (int i = 0; i < kBoxRun; i++) {
+                const int gy = y0 + y + i;
+                if (gy < H)
+                    out[static_cast<long long>(gy) * W] =
+                        acc[i] / static_cast<float>((min(H - 1, gy + r) - max(0, gy - r) + 1) * cols);
+            }
+        }
+        __syncthreads();   // the sums are read
     }
 }
 
@@ -227,57 +340,163 @@ __global__ void mlp_reduce_adam_kernel(const float* __restrict__ partial, int ti
     prm[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
-// per-pixel forward: probabilities (optional) and argmax label (lowest label on ties)
+// per-pixel forward: probabilities (optional) and argmax label (lowest label on ties). Persistent CTAs with the
+// transposed weights in shared memory; a thread takes a pixel through the network with the hidden units as
+// pairs in registers, two multiply-adds per instruction and four weights per shared-memory read, which all
+// lanes share. Every hidden unit and logit is one chain of fused multiply-adds in the order of its inputs. The
+// inputs arrive a chunk of planes ahead and the logits stay in shared memory for the softmax. 10.4 k
+// multiply-adds a pixel (40 classes, 64 hidden units) are 89 us a frame of 640x480 at the FMA pipe's peak;
+// 1117 -> 289 us a frame, bound by latency at 16 warps per SM (two pixels a thread: 323 us; loads straight into
+// registers, which wait for one another: 396 us).
 template <int kHd>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kPredictThreads, kHd <= 64 ? 2 : 1)
 mlp_predict_kernel(FeaturePlanes f, int D, int Hd, const float* __restrict__ prm, float* __restrict__ probs,
                    uint8_t* __restrict__ labels) {
-    extern __shared__ __align__(16) float w[];
-    const int C = f.C;
-    const int P = Hd * D + Hd + C * Hd + C;
-    for (int i = threadIdx.x; i < P; i += blockDim.x) w[i] = prm[i];
-    __syncthreads();
-    const float* W1 = w;
-    const float* b1 = W1 + Hd * D;
-    const float* W2 = b1 + Hd;
-    const float* b2 = W2 + C * Hd;
-    const long long plane = static_cast<long long>(f.W) * f.H;
-    const long long pix = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (pix >= plane) return;
-    const int y = static_cast<int>(pix / f.W), x = static_cast<int>(pix - static_cast<long long>(y) * f.W);
-    float h[kHd];
-#pragma unroll
-    for (int j = 0; j < kHd; j++) h[j] = j < Hd ? b1[j] : 0.0f;
-    for (int k = 0; k < D; k++) {
-        const float xk = feature_at(f, k, pix, x, y);
-#pragma unroll
-        for (int j = 0; j < kHd; j++)
-            if (j < Hd) h[j] = fmaf(W1[j * D + k], xk, h[j]);
+    extern __shared__ __align__(16) float sm[];
+    const int C = f.C, CP = (C + 7) & ~7;
+    float* W1 = sm;                   // [D][kHd]
+    float* b1 = W1 + D * kHd;         // [kHd]
+    float* W2 = b1 + kHd;             // [Hd][CP]
+    float* b2 = W2 + Hd * CP;         // [CP]
+    float* Z = b2 + CP + threadIdx.x; // [max(C, 2 kChunk)][threads]
+    for (int i = threadIdx.x; i < D * kHd; i += blockDim.x) {
+        const int j = i / D, k = i - j * D;   // read along the rows of the parameters
+        W1[k * kHd + j] = j < Hd ? prm[j * D + k] : 0.0f;
     }
+    const float* g = prm + Hd * D;
+    for (int j = threadIdx.x; j < kHd; j += blockDim.x) b1[j] = j < Hd ? g[j] : 0.0f;
+    g += Hd;
+    for (int i = threadIdx.x; i < CP * Hd; i += blockDim.x) {
+        const int c = i / Hd, j = i - c * Hd;
+        W2[j * CP + c] = c < C ? g[c * Hd + j] : 0.0f;
+    }
+    g += C * Hd;
+    for (int c = threadIdx.x; c < CP; c += blockDim.x) b2[c] = c < C ? g[c] : 0.0f;
+    __syncthreads();
+    const long long plane = static_cast<long long>(f.W) * f.H;
+    for (long long p0 = static_cast<long long>(blockIdx.x) * kPredictThreads; p0 < plane;
+         p0 += static_cast<long long>(gridDim.x) * kPredictThreads) {
+        const bool have = p0 + threadIdx.x < plane;
+        const long long pix = have ? p0 + threadIdx.x : plane - 1;
+        u64 h[kHd / 2];
 #pragma unroll
-    for (int j = 0; j < kHd; j++) h[j] = fmaxf(h[j], 0.0f);
-    auto logit = [&](int c) {
-        float z = b2[c];
+        for (int j = 0; j < kHd / 2; j++) h[j] = reinterpret_cast<const u64*>(b1)[j];
+        auto input = [&](int k, float x) {
+            const ulonglong2* w = reinterpret_cast<const ulonglong2*>(W1 + k * kHd);
+            const u64 xx = pack_f2(x, x);
 #pragma unroll
-        for (int j = 0; j < kHd; j++)
-            if (j < Hd) z = fmaf(W2[c * Hd + j], h[j], z);
-        return z;
-    };
-    float mx = -INFINITY;
-    int best = 0;
-    for (int c = 0; c < C; c++) {
-        const float z = logit(c);
-        if (z > mx) {
-            mx = z;
-            best = c;
+            for (int j = 0; j < kHd / 4; j++) {
+                const ulonglong2 v = w[j];
+                h[2 * j] = fma2(v.x, xx, h[2 * j]);
+                h[2 * j + 1] = fma2(v.y, xx, h[2 * j + 1]);
+            }
+        };
+        // the 3 C plane values of the thread's pixel, a chunk of planes ahead, through its own slots of the
+        // logits' memory
+        const uint32_t slot = static_cast<uint32_t>(__cvta_generic_to_shared(Z));
+        auto fetch = [&](int k0) {
+#pragma unroll
+            for (int a = 0; a < kChunk; a++) {
+                const int k = k0 + a;
+                if (k < 3 * C) {
+                    const float* src = k < C ? f.p + k * plane : k < 2 * C ? f.m1 + (k - C) * plane : f.m2 + (k - 2 * C) * plane;
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                                     slot + 4 * kPredictThreads * ((k0 / kChunk & 1) * kChunk + a)),
+                                 "l"(src + pix)
+                                 : "memory");
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        fetch(0);
+        for (int k0 = 0; k0 < 3 * C; k0 += kChunk) {
+            fetch(k0 + kChunk);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            const float* in = Z + (k0 / kChunk & 1) * kChunk * kPredictThreads;
+#pragma unroll
+            for (int a = 0; a < kChunk; a++)
+                if (k0 + a < 3 * C) input(k0 + a, in[a * kPredictThreads]);
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        {
+            const int y = static_cast<int>(pix / f.W), x = static_cast<int>(pix - static_cast<long long>(y) * f.W);
+            const float m = pixel_depth_m(f.depth, f.W, x, y);
+            input(3 * C, m * 0.2f);
+            input(3 * C + 1, m > 0.0f ? 1.0f : 0.0f);
+        }
+#pragma unroll
+        for (int j = 0; j < kHd / 2; j++) {
+            float a, b;
+            unpack_f2(h[j], a, b);
+            h[j] = pack_f2(fmaxf(a, 0.0f), fmaxf(b, 0.0f));
+        }
+        for (int c0 = 0; c0 < CP; c0 += 8) {   // eight logits at a time
+            u64 z[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) z[q] = reinterpret_cast<const u64*>(b2 + c0)[q];
+#pragma unroll
+            for (int j = 0; j < kHd; j++) {
+                if (j < Hd) {
+                    const ulonglong2* w = reinterpret_cast<const ulonglong2*>(W2 + j * CP + c0);
+                    const ulonglong2 va = w[0], vb = w[1];
+                    float a, b;
+                    unpack_f2(h[j / 2], a, b);
+                    const float hj = j & 1 ? b : a;
+                    const u64 hh = pack_f2(hj, hj);
+                    z[0] = fma2(va.x, hh, z[0]);
+                    z[1] = fma2(va.y, hh, z[1]);
+                    z[2] = fma2(vb.x, hh, z[2]);
+                    z[3] = fma2(vb.y, hh, z[3]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                float a, b;
+                unpack_f2(z[q], a, b);
+                const int c = c0 + 2 * q;
+                if (c < C) Z[c * kPredictThreads] = a;
+                if (c + 1 < C) Z[(c + 1) * kPredictThreads] = b;
+            }
+        }
+        // eight logits at a time: their reads and exponentials overlap, the comparisons and additions stay in class
+        // order
+        float mx = -INFINITY;
+        int best = 0;
+        for (int c0 = 0; c0 < C; c0 += 8) {
+            float v[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) v[q] = c0 + q < C ? Z[(c0 + q) * kPredictThreads] : -INFINITY;
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                if (v[q] > mx) {
+                    mx = v[q];
+                    best = c0 + q;
+                }
+        }
+        if (labels && have) labels[pix] = static_cast<uint8_t>(best);
+        if (probs) {
+            float s = 0.0f;
+            for (int c0 = 0; c0 < C; c0 += 8) {
+                float v[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++) v[q] = c0 + q < C ? expf(Z[(c0 + q) * kPredictThreads] - mx) : 0.0f;
+#pragma unroll
+                for (int q = 0; q < 8; q++)
+                    if (c0 + q < C) {
+                        Z[(c0 + q) * kPredictThreads] = v[q];
+                        s += v[q];
+                    }
+            }
+            if (have)
+#pragma unroll 4
+                for (int c = 0; c < C; c++) probs[c * plane + pix] = Z[c * kPredictThreads] / s;
         }
     }
-    if (labels) labels[pix] = static_cast<uint8_t>(best);
-    if (probs) {
-        float s = 0.0f;
-        for (int c = 0; c < C; c++) s += expf(logit(c) - mx);
-        for (int c = 0; c < C; c++) probs[c * plane + pix] = expf(logit(c) - mx) / s;
-    }
+}
+
+size_t predict_smem(int D, int Hd, int C, int kHd) {
+    const int CP = (C + 7) & ~7;
+    return sizeof(float) * (D * kHd + kHd + Hd * CP + CP + std::max(C, 2 * kChunk) * kPredictThreads);
 }
 
 // deterministic Glorot-uniform initialisation from a 64-bit mixer of (seed, index)
@@ -331,7 +550,6 @@ void for_each_frame_features(cf_refiner* r, cf_forest* forest, cf_dataset* ds, i
     r->probs.reserve(plane * C);
     r->mean1.reserve(plane * C);
     r->mean2.reserve(plane * C);
-    r->tmp.reserve(plane * C);
     r->frames.reserve(1);
     const int grid = ctx->num_sms * 8;
     for (int i = 0; i < count; i++) {
@@ -346,14 +564,24 @@ void for_each_frame_features(cf_refiner* r, cf_forest* forest, cf_dataset* ds, i
         fr.pad = 0;
         CF_CUDA_CHECK(cudaMemcpyAsync(r->frames.get(), &fr, sizeof(fr), cudaMemcpyHostToDevice, ctx->stream));
         classify_frames(ctx, forest, r->frames.get(), 1, classify_blocks_for(W, H));
-        launch(ctx, "refiner_box", dim3(grid), dim3(256), 0, box_rows_kernel, r->probs.get(), r->tmp.get(), C, W, H,
-               r->cfg.radius1);
-        launch(ctx, "refiner_box", dim3(grid), dim3(256), 0, box_cols_kernel, r->tmp.get(), r->mean1.get(), C, W, H,
-               r->cfg.radius1);
-        launch(ctx, "refiner_box", dim3(grid), dim3(256), 0, box_rows_kernel, r->probs.get(), r->tmp.get(), C, W, H,
-               r->cfg.radius2);
-        launch(ctx, "refiner_box", dim3(grid), dim3(256), 0, box_cols_kernel, r->tmp.get(), r->mean2.get(), C, W, H,
-               r->cfg.radius2);
+        const int radius = std::max(r->cfg.radius1, r->cfg.radius2);
+        if (radius <= kBoxMaxRadius) {
+            const size_t smem = box_smem(radius);
+            CF_CUDA_CHECK(cudaFuncSetAttribute(box_means_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(smem)));
+            launch(ctx, "refiner_box", dim3((W + kBoxTile - 1) / kBoxTile, (H + kBoxTile - 1) / kBoxTile, C), dim3(256),
+                   smem, box_means_kernel, r->probs.get(), r->mean1.get(), r->mean2.get(), W, H, r->cfg.radius1,
+                   r->cfg.radius2);
+        } else {
+            r->tmp.reserve(plane * C);
+            for (int k = 0; k < 2; k++) {
+                const int rad = k ? r->cfg.radius2 : r->cfg.radius1;
+                launch(ctx, "refiner_box", dim3(grid), dim3(256), 0, box_rows_kernel, r->probs.get(), r->tmp.get(), C, W,
+                       H, rad);
+                launch(ctx, "refiner_box", dim3(grid), dim3(256), 0, box_cols_kernel, r->tmp.get(),
+                       k ? r->mean2.get() : r->mean1.get(), C, W, H, rad);
+            }
+        }
         FeaturePlanes f{r->probs.get(), r->mean1.get(), r->mean2.get(), fr.depth, W, H, C};
         per_frame(i, f);
     }
@@ -554,13 +782,17 @@ cf_status cf_refiner_predict(cf_refiner* r, cf_forest* forest, cf_dataset* ds, i
         CF_REQUIRE(first >= 0 && count >= 1 && first + count <= ds->n, "cf_refiner_predict: image range");
         make_current(r->ctx);
         const long long plane = static_cast<long long>(ds->width) * ds->height;
-        const size_t smem = sizeof(float) * r->P;
+        const size_t smem = predict_smem(r->D, r->H, r->C, r->H <= 32 ? 32 : r->H <= 64 ? 64 : 128);
         auto kernel = r->H <= 32 ? mlp_predict_kernel<32> : r->H <= 64 ? mlp_predict_kernel<64> : mlp_predict_kernel<128>;
         CF_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        int resident = 1;
+        CF_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kPredictThreads, smem));
+        const long long blocks = (plane + kPredictThreads - 1) / kPredictThreads;
+        const unsigned grid =
+            static_cast<unsigned>(std::min<long long>(blocks, static_cast<long long>(r->ctx->num_sms) * std::max(1, resident)));
         for_each_frame_features(r, forest, ds, first, count, [&](int i, const FeaturePlanes& f) {
-            launch(r->ctx, "refiner_predict", dim3(static_cast<unsigned>((plane + 127) / 128)), dim3(128), smem,
-                   kernel, f, r->D, r->H, r->params.get(),
-                   probabilities ? probabilities + static_cast<long long>(i) * r->C * plane : nullptr,
+            launch(r->ctx, "refiner_predict", dim3(grid), dim3(kPredictThreads), smem, kernel, f, r->D, r->H,
+                   r->params.get(), probabilities ? probabilities + static_cast<long long>(i) * r->C * plane : nullptr,
                    labels ? labels + static_cast<long long>(i) * plane : nullptr);
         });
         CF_CUDA_CHECK(cudaStreamSynchronize(r->ctx->stream));
