@@ -22,7 +22,38 @@ void destroy_context_now(cf_context* ctx) {
     for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
     if (ctx->spare_trainer && ctx->spare_trainer_free) ctx->spare_trainer_free(ctx->spare_trainer);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
+    if (ctx->scratch_pool) cudaMemPoolDestroy(ctx->scratch_pool);
     delete ctx;
+}
+
+void* scratch_alloc(cf_context* ctx, size_t bytes, cudaStream_t stream) {
+    void* p = nullptr;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CF_CUDA_CHECK(cudaStreamIsCapturing(stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone) {   // a graph owns its memory
+        CF_CUDA_CHECK(cudaMallocAsync(&p, bytes, stream));
+        return p;
+    }
+    {
+        std::lock_guard<std::mutex> lock(ctx->mu);
+        if (ctx->scratch_pool == nullptr) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = ctx->device;
+            cudaMemPool_t pool = nullptr;
+            CF_CUDA_CHECK(cudaMemPoolCreate(&pool, &props));
+            uint64_t kept = cf_context::kScratchKept;
+            const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept);
+            if (e != cudaSuccess) {
+                cudaMemPoolDestroy(pool);
+                CF_CUDA_CHECK(e);
+            }
+            ctx->scratch_pool = pool;
+        }
+    }
+    CF_CUDA_CHECK(cudaMallocFromPoolAsync(&p, bytes, ctx->scratch_pool, stream));
+    return p;
 }
 
 void context_retain(cf_context* ctx) { ctx->refs++; }

@@ -7,9 +7,8 @@
 // wrapping 32-bit integers: box differences stay exact even where the reference's int
 // integral overflows (1280x960 frames at up to 5 m).
 //
-// Two passes: a warp-per-row inclusive scan of the five channels, then a thread-per-column
-// running sum down the rows. Traffic: 5 B/px read raw, 20 B/px written, then 20 B/px read and
-// written again.
+// Two passes: a warp-per-row inclusive scan of the five channels, then running sums down the columns in
+// segments. Traffic: 5 B/px read raw, 20 B/px written, then 20 B/px read and written again.
 #include <algorithm>
 #include <cstring>
 
@@ -19,8 +18,14 @@ namespace cf {
 
 namespace {
 
-constexpr int kRowWarps = 8;
+constexpr int kRowWarps = 4;
+constexpr int kColLanes = 32, kColSegments = 16, kColRun = 8;   // columns x row segments of a CTA, rows of a segment
 
+// Row prefix sums, a warp per row, 128 pixels a step with the next step's reads under way. A lane takes four
+// pixels; red and green, and blue and the valid count, share a word (sums of 128 pixels stay below 2^16), so a
+// step scans three words. kQuad: rows start on whole quads and the pointers are aligned (whole-word reads,
+// 16-byte writes); otherwise pixel by pixel.
+template <bool kQuad>
 __global__ void __launch_bounds__(kRowWarps * 32)
 integral_rows_kernel(const uint8_t* __restrict__ rgb, const uint16_t* __restrict__ depth, int count, int W, int H,
                      uint32_t* __restrict__ color_out, int2* __restrict__ depth_out) {
@@ -34,86 +39,171 @@ integral_rows_kernel(const uint8_t* __restrict__ rgb, const uint16_t* __restrict
     const uint16_t* src_d = depth + img * plane + static_cast<long long>(y) * W;
     uint32_t* dst_c = color_out + img * 3 * plane + static_cast<long long>(y) * W;
     int2* dst_d = depth_out + img * plane + static_cast<long long>(y) * W;
-    uint32_t carry[5] = {0, 0, 0, 0, 0};
-    for (int x0 = 0; x0 < W; x0 += 32) {
-        const int x = x0 + lane;
-        uint32_t v[5] = {0, 0, 0, 0, 0};
-        if (x < W) {
-            v[0] = src_rgb[x * 3 + 0];
-            v[1] = src_rgb[x * 3 + 1];
-            v[2] = src_rgb[x * 3 + 2];
-            v[3] = src_d[x];
-            v[4] = v[3] > 0 ? 1u : 0u;
+    struct Quad {
+        uint32_t c[3];   // twelve colour bytes
+        uint32_t d[2];   // four depths
+    };
+    auto read = [&](int x) {
+        Quad q = {};
+        if (kQuad) {
+            if (x < W) {
+                const uint32_t* c = reinterpret_cast<const uint32_t*>(src_rgb + 3 * x);
+                q.c[0] = __ldg(c);
+                q.c[1] = __ldg(c + 1);
+                q.c[2] = __ldg(c + 2);
+                const uint2 d = __ldg(reinterpret_cast<const uint2*>(src_d + x));
+                q.d[0] = d.x;
+                q.d[1] = d.y;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 12; k++)
+                if (x + k / 3 < W) q.c[k >> 2] |= static_cast<uint32_t>(src_rgb[3 * x + k]) << (8 * (k & 3));
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (x + k < W) q.d[k >> 1] |= static_cast<uint32_t>(src_d[x + k]) << (16 * (k & 1));
         }
+        return q;
+    };
+    uint32_t cr = 0, cg = 0, cb = 0, cd = 0, cn = 0;   // sums of the steps before
+    Quad next = read(4 * lane);
+    for (int x0 = 0; x0 < W; x0 += 128) {
+        const Quad q = next;
+        const int x = x0 + 4 * lane;
+        if (x0 + 128 < W) next = read(x + 128);
+        uint32_t rg[4], bn[4], d[4];
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-#pragma unroll
-            for (int c = 0; c < 5; c++) {
-                const uint32_t o = __shfl_up_sync(0xffffffffu, v[c], off);
-                if (lane >= off) v[c] += o;
+        for (int k = 0; k < 4; k++) {
+            auto byte = [&](int b) { return q.c[b >> 2] >> (8 * (b & 3)) & 255u; };
+            d[k] = q.d[k >> 1] >> (16 * (k & 1)) & 0xFFFFu;
+            rg[k] = byte(3 * k) | byte(3 * k + 1) << 16;
+            bn[k] = byte(3 * k + 2) | (d[k] > 0 ? 1u << 16 : 0u);
+            if (k > 0) {
+                rg[k] += rg[k - 1];
+                bn[k] += bn[k - 1];
+                d[k] += d[k - 1];
             }
         }
+        uint32_t srg = rg[3], sbn = bn[3], sd = d[3];
 #pragma unroll
-        for (int c = 0; c < 5; c++) v[c] += carry[c];
-        if (x < W) {
-            dst_c[x] = v[0];
-            dst_c[plane + x] = v[1];
-            dst_c[2 * plane + x] = v[2];
-            dst_d[x] = make_int2(static_cast<int>(v[3]), static_cast<int>(v[4]));
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t a = __shfl_up_sync(0xffffffffu, srg, off), b = __shfl_up_sync(0xffffffffu, sbn, off);
+            const uint32_t c = __shfl_up_sync(0xffffffffu, sd, off);
+            if (lane >= off) {
+                srg += a;
+                sbn += b;
+                sd += c;
+            }
         }
+        uint32_t r4[4], g4[4], b4[4];
+        int2 d4[4];
 #pragma unroll
-        for (int c = 0; c < 5; c++) carry[c] = __shfl_sync(0xffffffffu, v[c], 31);
+        for (int k = 0; k < 4; k++) {
+            const uint32_t prg = srg - rg[3] + rg[k], pbn = sbn - bn[3] + bn[k];
+            r4[k] = cr + (prg & 0xFFFFu);
+            g4[k] = cg + (prg >> 16);
+            b4[k] = cb + (pbn & 0xFFFFu);
+            d4[k] = make_int2(static_cast<int>(cd + sd - d[3] + d[k]), static_cast<int>(cn + (pbn >> 16)));
+        }
+        if (kQuad) {
+            if (x < W) {
+                *reinterpret_cast<uint4*>(dst_c + x) = make_uint4(r4[0], r4[1], r4[2], r4[3]);
+                *reinterpret_cast<uint4*>(dst_c + plane + x) = make_uint4(g4[0], g4[1], g4[2], g4[3]);
+                *reinterpret_cast<uint4*>(dst_c + 2 * plane + x) = make_uint4(b4[0], b4[1], b4[2], b4[3]);
+                int4* o = reinterpret_cast<int4*>(dst_d + x);
+                o[0] = make_int4(d4[0].x, d4[0].y, d4[1].x, d4[1].y);
+                o[1] = make_int4(d4[2].x, d4[2].y, d4[3].x, d4[3].y);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (x + k < W) {
+                    dst_c[x + k] = r4[k];
+                    dst_c[plane + x + k] = g4[k];
+                    dst_c[2 * plane + x + k] = b4[k];
+                    dst_d[x + k] = d4[k];
+                }
+        }
+        srg = __shfl_sync(0xffffffffu, srg, 31);
+        sbn = __shfl_sync(0xffffffffu, sbn, 31);
+        cr += srg & 0xFFFFu;
+        cg += srg >> 16;
+        cb += sbn & 0xFFFFu;
+        cn += sbn >> 16;
+        cd += __shfl_sync(0xffffffffu, sd, 31);
     }
 }
 
-__global__ void __launch_bounds__(256)
-integral_cols_kernel(int count, int W, int H, uint32_t* __restrict__ color, int2* __restrict__ depth) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const long long img = blockIdx.y;
-    if (x >= W || img >= count) return;
-    const long long plane = static_cast<long long>(W) * H;
-    uint32_t* c0 = color + img * 3 * plane + x;
-    int2* d0 = depth + img * plane + x;
-    uint32_t a0 = 0, a1 = 0, a2 = 0, a3 = 0, a4 = 0;
-    int y = 0;
-    for (; y + 4 <= H; y += 4) {
-        uint32_t r0[4], r1[4], r2[4];
-        int2 rd[4];
+// Column sums of one plane (three colours, then depth) in place: a CTA takes 32 columns, a thread 8 rows of one
+// of them at a time (all its reads under way together), the 16 segments of 128 rows are joined through shared
+// memory. A thread per column keeps too few reads in flight on one frame (66 us a frame of 640x480; 64 frames
+// 197 us).
+template <bool kDepth>
+__device__ __forceinline__ void sum_columns(void* column, bool ok, int W, int H) {
+    __shared__ uint32_t s_a[kColSegments][kColLanes], s_b[kColSegments][kColLanes];
+    uint32_t* c = static_cast<uint32_t*>(column);
+    int2* d = static_cast<int2*>(column);
+    const int seg = threadIdx.y;
+    uint32_t carry_a = 0, carry_b = 0;
+    for (int y0 = 0; y0 < H; y0 += kColSegments * kColRun) {
+        const int ya = y0 + seg * kColRun;
+        uint32_t va[kColRun], vb[kDepth ? kColRun : 1];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const long long o = static_cast<long long>(y + k) * W;
-            r0[k] = c0[o];
-            r1[k] = c0[plane + o];
-            r2[k] = c0[2 * plane + o];
-            rd[k] = d0[o];
+        for (int k = 0; k < kColRun; k++) {
+            va[k] = 0;
+            if constexpr (kDepth) vb[k] = 0;
+            if (ok && ya + k < H) {
+                const long long o = static_cast<long long>(ya + k) * W;
+                if constexpr (kDepth) {
+                    const int2 v = d[o];
+                    va[k] = static_cast<uint32_t>(v.x);
+                    vb[k] = static_cast<uint32_t>(v.y);
+                } else {
+                    va[k] = c[o];
+                }
+            }
         }
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const long long o = static_cast<long long>(y + k) * W;
-            a0 += r0[k];
-            a1 += r1[k];
-            a2 += r2[k];
-            a3 += static_cast<uint32_t>(rd[k].x);
-            a4 += static_cast<uint32_t>(rd[k].y);
-            reinterpret_cast<float*>(c0)[o] = __uint2float_rn(a0);
-            reinterpret_cast<float*>(c0)[plane + o] = __uint2float_rn(a1);
-            reinterpret_cast<float*>(c0)[2 * plane + o] = __uint2float_rn(a2);
-            d0[o] = make_int2(static_cast<int>(a3), static_cast<int>(a4));
+        for (int k = 1; k < kColRun; k++) {
+            va[k] += va[k - 1];
+            if constexpr (kDepth) vb[k] += vb[k - 1];
         }
+        __syncthreads();   // the previous step's sums are read
+        s_a[seg][threadIdx.x] = va[kColRun - 1];
+        if constexpr (kDepth) s_b[seg][threadIdx.x] = vb[kColRun - 1];
+        __syncthreads();
+        uint32_t before_a = carry_a, before_b = carry_b;
+#pragma unroll
+        for (int g = 0; g < kColSegments; g++) {
+            const uint32_t a = s_a[g][threadIdx.x];
+            before_a += g < seg ? a : 0u;
+            carry_a += a;
+            if constexpr (kDepth) {
+                const uint32_t b = s_b[g][threadIdx.x];
+                before_b += g < seg ? b : 0u;
+                carry_b += b;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kColRun; k++)
+            if (ok && ya + k < H) {
+                const long long o = static_cast<long long>(ya + k) * W;
+                if constexpr (kDepth) d[o] = make_int2(static_cast<int>(before_a + va[k]), static_cast<int>(before_b + vb[k]));
+                else reinterpret_cast<float*>(c)[o] = __uint2float_rn(before_a + va[k]);
+            }
     }
-    for (; y < H; y++) {
-        const long long o = static_cast<long long>(y) * W;
-        a0 += c0[o];
-        a1 += c0[plane + o];
-        a2 += c0[2 * plane + o];
-        const int2 rd = d0[o];
-        a3 += static_cast<uint32_t>(rd.x);
-        a4 += static_cast<uint32_t>(rd.y);
-        reinterpret_cast<float*>(c0)[o] = __uint2float_rn(a0);
-        reinterpret_cast<float*>(c0)[plane + o] = __uint2float_rn(a1);
-        reinterpret_cast<float*>(c0)[2 * plane + o] = __uint2float_rn(a2);
-        d0[o] = make_int2(static_cast<int>(a3), static_cast<int>(a4));
-    }
+}
+
+__global__ void __launch_bounds__(kColLanes * kColSegments, 2)
+integral_cols_kernel(int W, int H, uint32_t* __restrict__ color, int2* __restrict__ depth) {
+    const int strips = (W + kColLanes - 1) / kColLanes;
+    long long b = blockIdx.x;
+    const int x = static_cast<int>(b % strips) * kColLanes + threadIdx.x;
+    b /= strips;
+    const int p = static_cast<int>(b & 3);
+    const long long img = b >> 2, plane = static_cast<long long>(W) * H;
+    if (p < 3) sum_columns<false>(color + (img * 3 + p) * plane + x, x < W, W, H);
+    else sum_columns<true>(depth + img * plane + x, x < W, W, H);
 }
 
 // RGBDImage::resizeImage (image.cpp:450-475) applied to integral images: the w x h integrals go to the
@@ -154,11 +244,15 @@ void integrate_frames(cf_context* ctx, const uint8_t* rgb_dev, uint16_t* depth_d
     if (stream == nullptr) stream = ctx->stream;
     if (preprocess & kPreFillDepth) fill_depth_frames(ctx, depth_dev, count, W, H, stream);
     const long long rows = static_cast<long long>(count) * H;
+    auto aligned = [](const void* p, size_t n) { return reinterpret_cast<uintptr_t>(p) % n == 0; };
+    const bool quad = W % 4 == 0 && aligned(rgb_dev, 4) && aligned(depth_dev, 8) && aligned(color_out, 16) && aligned(depth_out, 16);
     launch_on(ctx, stream, "integral_rows", dim3(static_cast<unsigned>((rows + kRowWarps - 1) / kRowWarps)),
-           dim3(kRowWarps * 32), 0, integral_rows_kernel, rgb_dev, depth_dev, count, W, H,
-           reinterpret_cast<uint32_t*>(color_out), depth_out);
-    launch_on(ctx, stream, "integral_cols", dim3((W + 255) / 256, count), dim3(256), 0, integral_cols_kernel, count, W, H,
-           reinterpret_cast<uint32_t*>(color_out), depth_out);
+              dim3(kRowWarps * 32), 0, quad ? integral_rows_kernel<true> : integral_rows_kernel<false>, rgb_dev,
+              static_cast<const uint16_t*>(depth_dev), count, W, H, reinterpret_cast<uint32_t*>(color_out), depth_out);
+    const long long strips = (W + kColLanes - 1) / kColLanes;
+    launch_on(ctx, stream, "integral_cols", dim3(static_cast<unsigned>(strips * 4 * count)),
+              dim3(kColLanes, kColSegments), 0, integral_cols_kernel, W, H, reinterpret_cast<uint32_t*>(color_out),
+              depth_out);
     if (preprocess & kPreCieLab) lab_color_integral(ctx, rgb_dev, count, W, H, color_out, stream);
 }
 

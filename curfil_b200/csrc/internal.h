@@ -157,6 +157,10 @@ struct cf_context {
     // slot of at least 16 K evaluations, in multiples of 4 features, were 4-21 % faster on the levels
     // of that workload (more CTAs on one node's samples at a time, sharing their gathers in L2).
     static cf_eval_tuning default_tuning() { return cf_eval_tuning{16, 7168, 0, 3, 4, 2048.0f, 1, 16384, 1, 8192, 1}; }
+    // stream-ordered scratch of preprocessing; memory up to kScratchKept bytes stays with the pool between
+    // calls (the device's default pool gives everything back at each synchronisation)
+    cudaMemPool_t scratch_pool = nullptr;
+    static constexpr uint64_t kScratchKept = 256ull << 20;
     std::mutex mu;
     struct KernelEvents {
         std::vector<std::pair<cudaEvent_t, cudaEvent_t>> pending;
@@ -200,6 +204,10 @@ inline void launch(cf_context* ctx, const char* name, dim3 grid, dim3 block, siz
                    Args... args) {
     launch_on(ctx, ctx->stream, name, grid, block, smem, kernel, args...);
 }
+
+// `bytes` of device memory in stream order, to be given back with cudaFreeAsync on the same stream; valid inside
+// CUDA graph capture as well.
+void* scratch_alloc(cf_context* ctx, size_t bytes, cudaStream_t stream);
 
 inline void make_current(cf_context* ctx) { CF_CUDA_CHECK(cudaSetDevice(ctx->device)); }
 

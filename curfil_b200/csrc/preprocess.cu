@@ -17,22 +17,58 @@ namespace cf {
 
 namespace {
 
-__global__ void fill_depth_rows_kernel(uint16_t* __restrict__ d, long long rows, int W) {
-    const long long row = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+// The two row passes at once: a missing depth takes the next one to its right, or the row's last one where there
+// is none. A warp per row, from the right, 32 pixels a step (eight steps' reads under way together), the
+// nearest depth found by ballot. A thread per row with dependent reads took 140 us on four frames of 640x480.
+__global__ void __launch_bounds__(128)
+fill_depth_rows_kernel(uint16_t* __restrict__ d, long long rows, int W) {
+    constexpr int kAhead = 8;
+    const int lane = threadIdx.x & 31;
+    const long long row = blockIdx.x * 4ll + (threadIdx.x >> 5);
     if (row >= rows) return;
     uint16_t* r = d + row * W;
-    for (int x = W - 2; x >= 0; x--)
-        if (!r[x]) r[x] = r[x + 1];
-    for (int x = 1; x < W; x++)
-        if (!r[x]) r[x] = r[x - 1];
+    const int steps = (W + 31) / 32;
+    uint32_t carry = 0;   // the depth to the right of the step; first the row's last depth
+    for (int s = steps - 1; s >= 0 && carry == 0; s--) {
+        const int x = s * 32 + lane;
+        const uint32_t v = x < W ? r[x] : 0u;
+        const unsigned bal = __ballot_sync(0xffffffffu, v != 0);
+        if (bal) carry = __shfl_sync(0xffffffffu, v, 31 - __clz(bal));
+    }
+    if (carry == 0) return;   // no depth in this row
+    for (int s0 = steps - 1; s0 >= 0; s0 -= kAhead) {
+        uint32_t v[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; k++) {
+            const int x = (s0 - k) * 32 + lane;
+            v[k] = s0 >= k && x < W ? r[x] : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < kAhead; k++) {
+            if (s0 < k) break;
+            const int x = (s0 - k) * 32 + lane;
+            const unsigned bal = __ballot_sync(0xffffffffu, v[k] != 0);
+            const unsigned right = bal & (0xffffffffu << lane);
+            const uint32_t from = __shfl_sync(0xffffffffu, v[k], right ? __ffs(right) - 1 : lane);
+            const uint32_t filled = right ? from : carry;
+            if (x < W && v[k] == 0) r[x] = static_cast<uint16_t>(filled);
+            if (bal) carry = __shfl_sync(0xffffffffu, v[k], __ffs(bal) - 1);
+        }
+    }
 }
 
-__global__ void fill_depth_cols_kernel(uint16_t* __restrict__ d, int count, int W, int H) {
-    const long long col = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (col >= static_cast<long long>(count) * W) return;
-    const long long img = col / W;
-    const int x = static_cast<int>(col - img * W);
-    uint16_t* c = d + img * W * static_cast<long long>(H) + x;
+// The two column passes. After the row passes a row has all its depths or none, so the first of the CTA's own
+// columns tells whether any row of the frame is empty; if none is, there is nothing to do.
+__global__ void __launch_bounds__(256)
+fill_depth_cols_kernel(uint16_t* __restrict__ d, int W, int H) {
+    const int strips = (W + 255) / 256;
+    const long long img = blockIdx.x / strips;
+    const int x0 = static_cast<int>(blockIdx.x % strips) * 256, x = x0 + threadIdx.x;
+    uint16_t* frame = d + img * W * static_cast<long long>(H);
+    bool empty = false;
+    for (int y = threadIdx.x; y < H; y += 256) empty |= frame[static_cast<long long>(y) * W + x0] == 0;
+    if (!__syncthreads_or(empty) || x >= W) return;
+    uint16_t* c = frame + x;
     for (int y = 1; y < H; y++)
         if (!c[static_cast<long long>(y) * W]) c[static_cast<long long>(y) * W] = c[static_cast<long long>(y - 1) * W];
     for (int y = H - 2; y >= 0; y--)
@@ -61,29 +97,72 @@ __global__ void rgb_to_lab_kernel(const uint8_t* __restrict__ rgb, long long pix
     out[2 * plane] = static_cast<float>(200.0 * (fy - fz));
 }
 
-// row prefix sums in double of float planes (one thread per row of a plane)
-__global__ void prefix_rows_double_kernel(const float* __restrict__ in, double* __restrict__ out, long long rows, int W) {
-    const long long row = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (row >= rows) return;
+// Row prefix sums in double of float planes, each row summed from left to right. A warp takes 32 rows, a lane
+// summing one of them: tiles of 32 columns are read along the rows (the next tile's reads under way), turned in
+// shared memory, summed and turned back. A thread per row on its own reads and writes a line per value.
+constexpr int kPrefixWarps = 2;
+__global__ void __launch_bounds__(kPrefixWarps * 32)
+prefix_rows_double_kernel(const float* __restrict__ in, double* __restrict__ out, long long rows, int W) {
+    __shared__ float s_in[kPrefixWarps][32][33];
+    __shared__ double s_out[kPrefixWarps][32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long row0 = (blockIdx.x * static_cast<long long>(kPrefixWarps) + warp) * 32;
+    if (row0 >= rows) return;
+    const int n = static_cast<int>(min(32ll, rows - row0));
+    float next[32];
+    auto read = [&](int x) {
+#pragma unroll
+        for (int k = 0; k < 32; k++)
+            next[k] = k < n && x + lane < W ? __ldg(in + (row0 + k) * W + x + lane) : 0.0f;
+    };
+    read(0);
     double s = 0.0;
-    for (int x = 0; x < W; x++) {
-        s += static_cast<double>(in[row * W + x]);
-        out[row * W + x] = s;
+    for (int x0 = 0; x0 < W; x0 += 32) {
+#pragma unroll
+        for (int k = 0; k < 32; k++) s_in[warp][k][lane] = next[k];
+        __syncwarp();
+        if (x0 + 32 < W) read(x0 + 32);
+#pragma unroll
+        for (int k = 0; k < 32; k++) {
+            s += static_cast<double>(s_in[warp][lane][k]);
+            s_out[warp][lane][k] = s;
+        }
+        __syncwarp();
+#pragma unroll 8
+        for (int k = 0; k < 32; k++)
+            if (k < n && x0 + lane < W) out[(row0 + k) * W + x0 + lane] = s_out[warp][k][lane];
+        __syncwarp();
     }
 }
 
-// column prefix sums of the row sums (one thread per column of a plane), rounded to float
-__global__ void prefix_cols_float_kernel(const double* __restrict__ in, float* __restrict__ out, long long planes,
-                                         int W, int H) {
+// Column prefix sums of the row sums, each column summed from top to bottom and rounded to float: a thread per
+// column, 32 rows a step with the next step's reads under way.
+__global__ void __launch_bounds__(64)
+prefix_cols_float_kernel(const double* __restrict__ in, float* __restrict__ out, long long planes, int W, int H) {
+    constexpr int kRun = 32;
     const long long col = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (col >= planes * W) return;
     const long long pl = col / W;
     const int x = static_cast<int>(col - pl * W);
     const long long base = pl * W * static_cast<long long>(H) + x;
+    double next[kRun];
+    auto read = [&](int y) {
+#pragma unroll
+        for (int k = 0; k < kRun; k++) next[k] = y + k < H ? __ldg(in + base + static_cast<long long>(y + k) * W) : 0.0;
+    };
+    read(0);
     double s = 0.0;
-    for (int y = 0; y < H; y++) {
-        s += in[base + static_cast<long long>(y) * W];
-        out[base + static_cast<long long>(y) * W] = static_cast<float>(s);
+    for (int y0 = 0; y0 < H; y0 += kRun) {
+        double v[kRun];
+#pragma unroll
+        for (int k = 0; k < kRun; k++) v[k] = next[k];
+        if (y0 + kRun < H) read(y0 + kRun);
+#pragma unroll
+        for (int k = 0; k < kRun; k++)
+            if (y0 + k < H) {
+                s += v[k];
+                out[base + static_cast<long long>(y0 + k) * W] = static_cast<float>(s);
+            }
     }
 }
 
@@ -115,14 +194,29 @@ __global__ void prefix_cols_int_kernel(int32_t* __restrict__ d, long long planes
 
 }  // namespace
 
+namespace {
+
+void launch_prefix_rows(cf_context* ctx, cudaStream_t stream, const char* name, const float* in, double* out, long long rows,
+                        int W) {
+    launch_on(ctx, stream, name, dim3(static_cast<unsigned>((rows + 32 * kPrefixWarps - 1) / (32 * kPrefixWarps))),
+              dim3(32 * kPrefixWarps), 0, prefix_rows_double_kernel, in, out, rows, W);
+}
+
+void launch_prefix_cols(cf_context* ctx, cudaStream_t stream, const char* name, const double* in, float* out,
+                        long long planes, int W, int H) {
+    launch_on(ctx, stream, name, dim3(static_cast<unsigned>((planes * W + 63) / 64)), dim3(64), 0, prefix_cols_float_kernel,
+              in, out, planes, W, H);
+}
+
+}  // namespace
+
 void fill_depth_frames(cf_context* ctx, uint16_t* depth, int count, int W, int H, cudaStream_t stream) {
     if (stream == nullptr) stream = ctx->stream;
     const long long rows = static_cast<long long>(count) * H;
-    launch_on(ctx, stream, "fill_depth", dim3(static_cast<unsigned>((rows + 127) / 128)), dim3(128), 0,
+    launch_on(ctx, stream, "fill_depth", dim3(static_cast<unsigned>((rows + 3) / 4)), dim3(128), 0,
               fill_depth_rows_kernel, depth, rows, W);
-    const long long cols = static_cast<long long>(count) * W;
-    launch_on(ctx, stream, "fill_depth", dim3(static_cast<unsigned>((cols + 127) / 128)), dim3(128), 0,
-              fill_depth_cols_kernel, depth, count, W, H);
+    launch_on(ctx, stream, "fill_depth", dim3(static_cast<unsigned>((W + 255) / 256 * static_cast<long long>(count))),
+              dim3(256), 0, fill_depth_cols_kernel, depth, W, H);
 }
 
 void rgb_to_lab(cf_context* ctx, const uint8_t* rgb, int count, int W, int H, float* lab, cudaStream_t stream) {
@@ -138,20 +232,15 @@ void lab_color_integral(cf_context* ctx, const uint8_t* rgb, int count, int W, i
     if (stream == nullptr) stream = ctx->stream;
     const long long plane = static_cast<long long>(W) * H;
     const long long planes = 3LL * count;
-    // stream-ordered scratch (valid inside CUDA graph capture as well)
-    float* lab = nullptr;
-    double* rows = nullptr;
-    CF_CUDA_CHECK(cudaMallocAsync(reinterpret_cast<void**>(&lab), sizeof(float) * planes * plane, stream));
-    CF_CUDA_CHECK(cudaMallocAsync(reinterpret_cast<void**>(&rows), sizeof(double) * planes * plane, stream));
+    const size_t lab_bytes = (sizeof(float) * planes * plane + 255) & ~size_t(255);
+    const size_t bytes = lab_bytes + sizeof(double) * planes * plane;
+    unsigned char* scratch = static_cast<unsigned char*>(scratch_alloc(ctx, bytes, stream));
+    float* lab = reinterpret_cast<float*>(scratch);
+    double* rows = reinterpret_cast<double*>(scratch + lab_bytes);
     rgb_to_lab(ctx, rgb, count, W, H, lab, stream);
-    const long long nrows = planes * H;
-    launch_on(ctx, stream, "lab_integral", dim3(static_cast<unsigned>((nrows + 127) / 128)), dim3(128), 0,
-              prefix_rows_double_kernel, lab, rows, nrows, W);
-    const long long ncols = planes * W;
-    launch_on(ctx, stream, "lab_integral", dim3(static_cast<unsigned>((ncols + 127) / 128)), dim3(128), 0,
-              prefix_cols_float_kernel, rows, color_out, planes, W, H);
-    CF_CUDA_CHECK(cudaFreeAsync(rows, stream));
-    CF_CUDA_CHECK(cudaFreeAsync(lab, stream));
+    launch_prefix_rows(ctx, stream, "lab_integral", lab, rows, planes * H, W);
+    launch_prefix_cols(ctx, stream, "lab_integral", rows, color_out, planes, W, H);
+    CF_CUDA_CHECK(cudaFreeAsync(scratch, stream));
 }
 
 }  // namespace cf
@@ -211,11 +300,8 @@ cf_status cf_integrate_planes(cf_context* ctx, int count, int width, int height,
             CF_CUDA_CHECK(cudaMemcpyAsync(depth_integral, depth, sizeof(int32_t) * dplanes * plane,
                                           cudaMemcpyDeviceToDevice, st));
         }
-        const long long crows = cplanes * height, ccols = cplanes * width;
-        launch(ctx, "integral_planes", dim3(static_cast<unsigned>((crows + 127) / 128)), dim3(128), 0,
-               prefix_rows_double_kernel, c_in, rows.get(), crows, width);
-        launch(ctx, "integral_planes", dim3(static_cast<unsigned>((ccols + 127) / 128)), dim3(128), 0,
-               prefix_cols_float_kernel, rows.get(), c_out, cplanes, width, height);
+        launch_prefix_rows(ctx, st, "integral_planes", c_in, rows.get(), cplanes * height, width);
+        launch_prefix_cols(ctx, st, "integral_planes", rows.get(), c_out, cplanes, width, height);
         const long long drows = dplanes * height, dcols = dplanes * width;
         launch(ctx, "integral_planes", dim3(static_cast<unsigned>((drows + 127) / 128)), dim3(128), 0,
                prefix_rows_int_kernel, dep, drows, width);
