@@ -102,7 +102,8 @@ struct EvalArgs {
     int staged_f0 = 0;
     const long long* row_base = nullptr;
     const uint8_t* row_label = nullptr;
-    const int* staged_flip_both = nullptr;   // nonzero: a sample of the level has flip 2
+    const uint8_t* row_both = nullptr;   // where samples have flip 2: row r's flipped bins are those of row
+    long long both_rows = 0;             // both_rows + r if row_both[r]
     // fused search over a copy of the samples sorted by (node, frame, Morton code): node n's samples
     // are rows row_base[n] .. of it; nullptr: the level's own array
     const Sample* sorted_samples = nullptr;
@@ -333,9 +334,8 @@ level_eval_kernel(EvalArgs a) {
 
         for (int f0 = item.f_begin; f0 < item.f_end; f0 += ft) {
             const int nf = min(ft, item.f_end - f0);
-            // ---- stage the tile (the parameters and thresholds only where responses are computed: not
-            // for staged bins unless a sample of the level is evaluated both ways)
-            const bool need_thr = !a.staged || *a.staged_flip_both;
+            // ---- stage the tile (the parameters and thresholds only where responses are computed)
+            const bool need_thr = !a.staged;
             for (int i = tid; i < nf && need_thr; i += blockDim.x) s_params[i] = make_eval_feat(a.packs[f0 + i]);
             const float* g_thr = a.sorted_thr + static_cast<long long>(f0) * T;
             if (!need_thr) {
@@ -363,8 +363,7 @@ level_eval_kernel(EvalArgs a) {
                 // segments, so a tile reads one contiguous run. WL lanes (nw rounded up to a power of
                 // two) take one sample, a lane one word, i.e. four bins, and each lane kStagedUnroll
                 // samples per step so that several loads are in flight. A sample evaluated both ways
-                // (flip 2) has its unflipped bin staged; the flipped one is computed here by the
-                // sample's first lane.
+                // (flip 2) has a second row with its flipped bins.
                 const int off = f0 - a.staged_f0;
                 const int o = off & 31;
                 const int lead = o & 3;
@@ -376,26 +375,20 @@ level_eval_kernel(EvalArgs a) {
                 const long long row0 = a.row_base[item.node] + (sbase - nd.start);
                 const uint8_t* rows = a.staged + ((static_cast<long long>(off >> 5) * a.staged_rows + row0) << 5) + (o - lead);
                 for (int s0 = warp * (32 / WL); s0 < N; s0 += kStagedUnroll * step) {   // trip count uniform in a warp
-                    uint32_t v[kStagedUnroll];
-                    int lid[kStagedUnroll], flip[kStagedUnroll];
-                    bool act[kStagedUnroll];
-                    Sample smp[kStagedUnroll];
+                    uint32_t v[kStagedUnroll], v2[kStagedUnroll];
+                    int lid[kStagedUnroll];
+                    bool act[kStagedUnroll], two[kStagedUnroll];
 #pragma unroll
                     for (int u = 0; u < kStagedUnroll; u++) {
                         const int s = s0 + js + u * step;
                         const bool sv = s < N;
                         const int sc = sv ? s : N - 1;
                         act[u] = sv && wi < nw;
-                        v[u] = act[u] ? __ldg(reinterpret_cast<const uint32_t*>(rows + (static_cast<long long>(sc) << 5)) + wi)
-                                      : 0u;
-                        if (need_thr) {   // a sample of the level has flip 2: the whole sample
-                            smp[u] = a.samples[sbase + sc];
-                            lid[u] = smp[u].label;
-                            flip[u] = sv && wi == 0 ? smp[u].flip : 0;
-                        } else {
-                            lid[u] = a.row_label[row0 + sc];
-                            flip[u] = 0;
-                        }
+                        const uint8_t* at = rows + (static_cast<long long>(sc) << 5);
+                        v[u] = act[u] ? __ldg(reinterpret_cast<const uint32_t*>(at) + wi) : 0u;
+                        lid[u] = a.row_label[row0 + sc];
+                        two[u] = a.row_both && act[u] && a.row_both[row0 + sc];
+                        v2[u] = two[u] ? __ldg(reinterpret_cast<const uint32_t*>(at + (a.both_rows << 5)) + wi) : 0u;
                     }
 #pragma unroll
                     for (int u = 0; u < kStagedUnroll; u++) {
@@ -408,21 +401,16 @@ level_eval_kernel(EvalArgs a) {
                                                 ok ? (f * cp + lid[u]) * T1 + static_cast<int>((v[u] >> (8 * b)) & 0xffu) : -1);
                         }
                     }
-                    bool both = false;
+                    if (a.row_both) {
 #pragma unroll
-                    for (int u = 0; u < kStagedUnroll; u++) both = both || flip[u] == 2;
-                    if (__any_sync(kFull, both)) {
+                        for (int u = 0; u < kStagedUnroll; u++)
 #pragma unroll
-                        for (int u = 0; u < kStagedUnroll; u++) {
-                            const EvalPixel px = make_eval_pixel(a.ds, smp[u]);
-                            for (int f = 0; f < nf; f++) {
-                                const SortedBins<kPad> sorted{s_thr + f * TPS, T};
-                                const int key = flip[u] == 2
-                                                    ? (f * cp + lid[u]) * T1 + feature_bin(px, W, H, s_params[f], true, sorted)
-                                                    : -1;
-                                bin_increment<kAgg>(s_bins, key);
+                            for (int b = 0; b < 4; b++) {
+                                const int f = 4 * wi + b - lead;
+                                const bool ok = two[u] && f >= 0 && f < nf;
+                                bin_increment<kAgg>(
+                                    s_bins, ok ? (f * cp + lid[u]) * T1 + static_cast<int>((v2[u] >> (8 * b)) & 0xffu) : -1);
                             }
-                        }
                     }
                 }
             } else if constexpr (kGrouped) {
@@ -1220,7 +1208,7 @@ void LevelEvaluator::order_rows(cf_context* ctx, const DsView& ds, const Sample*
 // ------------------------------------------------------------------------------------------------
 void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* samples, const NodeDesc* nodes_dev,
                               const uint32_t* node_hist_dev, int M, const std::vector<int>& node_counts, int C,
-                              const LevelFeatures& lf, cf_split* splits_dev, uint32_t* dump_left) {
+                              const LevelFeatures& lf, cf_split* splits_dev, bool may_flip_both, uint32_t* dump_left) {
     const int F = lf.F, T = lf.T;
     CF_REQUIRE(C >= 1 && C <= 256, "number of classes must be in [1, 256]");
     CF_REQUIRE(T >= 1 && T <= 4096, "number of thresholds must be in [1, 4096]");
@@ -1228,13 +1216,33 @@ void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* s
     tuning = EvalTuning::of(ctx);
     const int slots = ctx->num_sms * tuning.ctas_per_sm;
     const bool sharded = shard.world > 1;
-    // staged bins: where the integral images do not fit in L2 (or on every level with stage_bins = 2);
-    // the bins are bytes (T <= 255)
+    // staged bins: on every level where the integral images do not fit in L2, and otherwise where the level is
+    // large enough to pay for the two passes' preparation (kStageMinEvals) and the gather kernel serves it; with
+    // stage_bins = 2 on every level. The bins are bytes (T <= 255)
     long long rows = 0;
     for (int c : node_counts) rows += c;
+    const long long table_rows = may_flip_both ? 2 * rows : rows;
     const size_t frame_bytes = static_cast<size_t>(ds.n) * ds.plane * (3 * sizeof(float) + sizeof(int2));
-    const bool stage = tuning.stage_bins != 0 && !sharded && T <= 255 && rows > 0 && rows < INT_MAX &&
-                       (tuning.stage_bins == 2 || frame_bytes > ctx->l2_bytes);
+    bool stage = tuning.stage_bins != 0 && !sharded && T <= 255 && rows > 0 && table_rows < INT_MAX &&
+                 (tuning.stage_bins == 2 || frame_bytes > ctx->l2_bytes ||
+                  (BinStager::gathers(ds, T) && (table_rows * F >= kStageMinEvals ||
+                                                 (table_rows * F >= kStageMinEvals / 4 && F >= 256 && M >= 64))));
+    int stage_chunk = 0, n_chunks = 0;
+    if (stage) {
+        // feature chunks of whole 32-feature tiles whose table fits stage_max_mb, as even as possible
+        const long long f_pad = (F + kStageTile - 1) / kStageTile * kStageTile;
+        const long long max_bytes = static_cast<long long>(tuning.stage_max_mb) << 20;
+        const long long tiles_max = std::max<long long>(1, max_bytes / rows / kStageTile);
+        n_chunks = static_cast<int>((f_pad / kStageTile + tiles_max - 1) / tiles_max);
+        stage_chunk = static_cast<int>((f_pad / kStageTile + n_chunks - 1) / n_chunks) * kStageTile;
+        n_chunks = (F + stage_chunk - 1) / stage_chunk;
+        try {
+            stage_.reserve(static_cast<size_t>(table_rows) * stage_chunk);
+        } catch (const Error& e) {
+            if (e.code != CF_ERR_OOM || !may_flip_both) throw;
+            stage = false;   // no room for the second half of the table: one pass
+        }
+    }
     // the staged search reads bytes instead of gathering, so it needs no L1: a larger histogram and
     // tiles of up to 32 features, and items of whole 32-feature rows (fewer, larger items: no CTAs
     // need to share a node's gathers)
@@ -1259,19 +1267,8 @@ void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* s
     const int max_groups = static_cast<int>(kMaxChunkGroupBytes / (sizeof(uint32_t) * static_cast<size_t>(budget)));
     plan_level_items(node_counts, F, plan, slots, h_items_, h_range_, h_order_, chunk_features, &n_groups,
                      max_groups);
-    int stage_chunk = 0, n_chunks = 0;
-    size_t stage_bytes = 0;
-    if (stage) {
-        // feature chunks of whole 32-feature tiles whose table fits stage_max_mb, as even as possible
-        const long long f_pad = (F + kStageTile - 1) / kStageTile * kStageTile;
-        const long long max_bytes = static_cast<long long>(tuning.stage_max_mb) << 20;
-        const long long tiles_max = std::max<long long>(1, max_bytes / rows / kStageTile);
-        n_chunks = static_cast<int>((f_pad / kStageTile + tiles_max - 1) / tiles_max);
-        stage_chunk = static_cast<int>((f_pad / kStageTile + n_chunks - 1) / n_chunks) * kStageTile;
-        n_chunks = (F + stage_chunk - 1) / stage_chunk;
-        stage_bytes = static_cast<size_t>(rows) * stage_chunk;
+    if (stage)
         split_items_into_chunks(node_counts, stage_chunk, n_chunks, h_items_, h_range_, h_order_, h_chunk_begin_);
-    }
     last_stage_chunks = stage ? n_chunks : 0;
     const int n_items = static_cast<int>(h_items_.size());
     // this process's items: every position of the work order, or positions rank, rank + world, ...
@@ -1334,15 +1331,15 @@ void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* s
         CF_CUDA_CHECK(cudaMemsetAsync(queue_.get(), 0, sizeof(int) * n_chunks, ctx->stream));
         set_row_base(ctx, M, node_counts);
         row_label_.reserve(rows);
-        flip_both_.reserve(1);
-        stager_.prepare(ctx, ds, samples, nodes_dev, M, row_base_.get(), rows, lf, stage_chunk, n_chunks, row_label_.get(),
-                        flip_both_.get());
-        stage_.reserve(stage_bytes);
+        if (may_flip_both) row_both_.reserve(rows);
+        stager_.prepare(ctx, ds, samples, nodes_dev, M, row_base_.get(), rows, may_flip_both, lf, stage_chunk, n_chunks,
+                        row_label_.get(), row_both_.get());
         args.staged = stage_.get();
-        args.staged_rows = rows;
+        args.staged_rows = table_rows;
         args.row_label = row_label_.get();
         args.row_base = row_base_.get();
-        args.staged_flip_both = flip_both_.get();
+        args.row_both = may_flip_both ? row_both_.get() : nullptr;
+        args.both_rows = rows;
         for (int c = 0; c < n_chunks; c++) {
             stager_.run(ctx, ds, samples, lf, c, stage_.get());
             args.staged_f0 = c * stage_chunk;

@@ -83,6 +83,11 @@ void plan_level_items(const std::vector<int>& node_counts, int F, const EvalTuni
 constexpr int kStagedFeatures = 32;           // features per tile at most
 constexpr int kStagedBinsWords = 12288;       // histogram words per CTA
 constexpr double kStagedItemsPerSlot = 64.0;  // work items per resident CTA at most (16 and 256: the same)
+// Frames within L2: sample-feature pairs from which a level is staged; a quarter of that for levels of many nodes
+// and features, whose one-pass items are small. 24 frames 313x235, one pass against two, all in us: 2.4 M pairs in
+// one node 241 / 316, in 97 nodes 533 / 467, in 2000 nodes 1503 / 1088; 6 M (100 features) 460 / 481; 9.6 M in one
+// node 492 / 445; 30 M 877 / 773; 120 M in 97 nodes 3288 / 2208.
+constexpr long long kStageMinEvals = 1ll << 23;
 // Splits every item at the chunk boundaries (multiples of `chunk` features) and orders the items
 // chunk by chunk, largest first within a chunk; chunk_begin[c] is the first order position of chunk c.
 void split_items_into_chunks(const std::vector<int>& node_counts, int chunk, int n_chunks,
@@ -92,10 +97,11 @@ void split_items_into_chunks(const std::vector<int>& node_counts, int chunk, int
 class LevelEvaluator {
 public:
     // nodes_dev / node_hist_dev: M node descriptors and [M][C] histograms on the device;
-    // node_counts: the M sample counts on the host (for work-item sizing).
+    // node_counts: the M sample counts on the host (for work-item sizing); may_flip_both: false where no sample
+    // of the level has flip 2.
     void evaluate(cf_context* ctx, const DsView& ds, const Sample* samples, const NodeDesc* nodes_dev,
                   const uint32_t* node_hist_dev, int M, const std::vector<int>& node_counts, int C,
-                  const LevelFeatures& lf, cf_split* splits_dev, uint32_t* dump_left = nullptr);
+                  const LevelFeatures& lf, cf_split* splits_dev, bool may_flip_both, uint32_t* dump_left = nullptr);
     EvalTuning tuning;            // the context's tuning at the last evaluate call
     int64_t last_items = 0;
     int last_stage_chunks = 0;    // feature chunks of the staged bins at the last call (0: not staged)
@@ -131,7 +137,7 @@ private:
     DevArray<long long> row_base_;    // [M + 1] first row of each node
     DevArray<int> row_pos_;           // [rows] position of each row's sample in the level's array
     DevArray<uint8_t> row_label_;     // [rows] label of each row's sample
-    DevArray<int> flip_both_;         // set when a sample of the level has flip 2
+    DevArray<uint8_t> row_both_;      // [rows] 1 where a row's sample has flip 2
     DevArray<Sample> sorted_samples_; // [rows] the level's samples sorted by (node, frame, Morton code)
     DevArray<unsigned long long> pixel_key_, pixel_key_sorted_;   // (node, frame, Morton code of y, x) of each row
     DevArray<int> row_ids_, frame_order_;   // rows, and rows in key order

@@ -34,8 +34,8 @@ constexpr int kThreads = 512;         // 16 warps: kRows / 32 groups of lanes x 
 constexpr int kCtasPerSm = 2;         // 64 registers; the shared memory left over is L1
 constexpr int kRows = 64;             // samples of a CTA (32: idle lanes of the tag pipe; 128, 256: 2-8 % slower)
 constexpr int kTileFeatures = 128;    // features staged at a time
-constexpr int kMorton = 32;           // key bits below the frame
-constexpr int kGeneralTile = 64;      // features per work item of the general kernel
+constexpr int kGeneralTile = 16;      // features per work item of the general kernel, which mostly takes few rows:
+                                      // 64 kept one CTA 45-90 us on the few rows of a small level
 constexpr int kGeneralCtasPerSm = 3;
 
 // Floats of a feature's row: eight parameters, +-2^23 with the sign of each offset, then the ascending
@@ -50,81 +50,72 @@ __device__ __forceinline__ int pair_code(const FeatParams& f) {
     return f.ch1 < 3 && f.ch2 < 3 ? 1 + f.ch1 * 3 + f.ch2 : kStageCodes - 1;
 }
 
-// The largest magnitude a candidate of the level scales by a depth.
-__global__ void stage_reach_kernel(int F, const FeatParams* __restrict__ packs, int* __restrict__ reach) {
-    int m = 1;
-    for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < F; f += gridDim.x * blockDim.x) {
-        const FeatParams p = packs[f];
-        m = max(m, max(max(abs(p.o1x), abs(p.o1y)), max(abs(p.o2x), abs(p.o2y))));
-        m = max(m, max(max(abs(p.r1x), abs(p.r1y)), max(abs(p.r2x), abs(p.r2y))));
-    }
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) atomicMax(reach, m);
-}
-
-__global__ void stage_feature_rows_kernel(int F, int T, int row, const FeatParams* __restrict__ packs,
-                                          const float* __restrict__ sorted_thr, float* __restrict__ out) {
-    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    const int f = static_cast<int>(i / row), k = static_cast<int>(i - static_cast<long long>(f) * row);
-    if (f >= (F + kStageUnit - 1) / kStageUnit * kStageUnit) return;
-    float v;
-    if (k < kRowParams) {
-        const FeatParams p = f < F ? packs[f] : FeatParams{};   // whole units: the rows past F hold zeros
-        const int8_t par[8] = {p.o1x, p.o1y, p.o2x, p.o2y, p.r1x, p.r1y, p.r2x, p.r2y};
-        v = k < 8 ? static_cast<float>(par[k]) : par[k - 8] < 0 ? -8388608.0f : 8388608.0f;
-    } else {
-        const int t = k - kRowParams;
-        v = t < T && f < F ? sorted_thr[static_cast<long long>(f) * T + t] : INFINITY;
-    }
-    out[i] = v;
-}
-
-// One CTA per feature chunk: the 8-feature blocks of every code (a block with features of several codes is
-// listed in each, with the mask of its features).
+// The candidates laid out for the kernels below. Blocks past `row_blocks` take a feature chunk each: the
+// 8-feature blocks of every code (a block with features of several codes is listed in each, with the mask of its
+// features), by one warp in block order. The others write the feature rows (row = 0: none) and find the largest
+// magnitude that a candidate of the level scales by a depth.
 __global__ void __launch_bounds__(256)
-stage_units_kernel(int F, int chunk, int cap, const FeatParams* __restrict__ packs, uint32_t* __restrict__ units,
-                   int* __restrict__ unit_count) {
-    __shared__ int s_n[kStageCodes];
-    const int f0 = blockIdx.x * chunk, n = min(chunk, F - f0);
-    if (threadIdx.x < kStageCodes) s_n[threadIdx.x] = 0;
-    __syncthreads();
+stage_plan_kernel(int F, int T, int row, int row_blocks, int chunk, int cap, const FeatParams* __restrict__ packs,
+                  const float* __restrict__ sorted_thr, float* __restrict__ rows, int* __restrict__ reach,
+                  uint32_t* __restrict__ units, int* __restrict__ unit_count) {
     const int lane = threadIdx.x & 31;
+    if (static_cast<int>(blockIdx.x) < row_blocks) {
+        const long long i = blockIdx.x * 256ll + threadIdx.x;
+        const int per = max(row, kRowParams);
+        const int f = static_cast<int>(i / per), k = static_cast<int>(i - static_cast<long long>(f) * per);
+        float v = 0.0f;
+        if (f < (F + kStageUnit - 1) / kStageUnit * kStageUnit) {
+            if (k < kRowParams) {
+                const FeatParams p = f < F ? packs[f] : FeatParams{};   // whole units: the rows past F hold zeros
+                const int8_t par[8] = {p.o1x, p.o1y, p.o2x, p.o2y, p.r1x, p.r1y, p.r2x, p.r2y};
+                v = k < 8 ? static_cast<float>(par[k]) : par[k - 8] < 0 ? -8388608.0f : 8388608.0f;
+            } else {
+                const int t = k - kRowParams;
+                v = t < T && f < F ? sorted_thr[static_cast<long long>(f) * T + t] : INFINITY;
+            }
+            if (row > 0) rows[i] = v;
+        }
+        const int m = __reduce_max_sync(0xffffffffu, k < 8 ? static_cast<int>(fabsf(v)) : 0);
+        if (lane == 0) atomicMax(reach, m);
+        return;
+    }
+    const int ch = static_cast<int>(blockIdx.x) - row_blocks;
+    const int f0 = ch * chunk, n = min(chunk, F - f0);
     const int blocks = (n + kStageUnit - 1) / kStageUnit;
-    uint32_t* mine = units + static_cast<long long>(blockIdx.x) * kStageCodes * cap;
-    if (threadIdx.x < 32) {   // one warp, in block order
-        for (int b0 = 0; b0 < blocks; b0 += 32) {
-            const int b = b0 + lane;
-            u64 codes = ~0ull;   // 4 bits per feature, 15: none
-            for (int j = 0; j < kStageUnit; j++) {
-                const int f = b * kStageUnit + j;
-                const u64 c = b < blocks && f < n ? pair_code(packs[f0 + f]) : 15;
-                codes = (codes & ~(15ull << (4 * j))) | (c << (4 * j));
-            }
-            for (int c = 0; c < kStageCodes; c++) {
-                uint32_t mask = 0;
-                for (int j = 0; j < kStageUnit; j++)
-                    if (((codes >> (4 * j)) & 15ull) == static_cast<u64>(c)) mask |= 1u << j;
-                const unsigned bal = __ballot_sync(0xffffffffu, mask != 0);
-                const int at = s_n[c] + __popc(bal & ((1u << lane) - 1u));
-                if (mask) mine[c * cap + at] = static_cast<uint32_t>(b) << 8 | mask;
-                __syncwarp();
-                if (lane == 0) s_n[c] += __popc(bal);
-                __syncwarp();
-            }
+    uint32_t* mine = units + static_cast<long long>(ch) * kStageCodes * cap;
+    if (threadIdx.x >= 32) return;
+    int count = 0;   // of code `lane`
+    for (int b0 = 0; b0 < blocks; b0 += 32) {
+        const int b = b0 + lane;
+        u64 codes = ~0ull;   // 4 bits per feature, 15: none
+        for (int j = 0; j < kStageUnit; j++) {
+            const int f = b * kStageUnit + j;
+            const u64 c = b < blocks && f < n ? pair_code(packs[f0 + f]) : 15;
+            codes = (codes & ~(15ull << (4 * j))) | (c << (4 * j));
+        }
+        for (int c = 0; c < kStageCodes; c++) {
+            uint32_t mask = 0;
+            for (int j = 0; j < kStageUnit; j++)
+                if (((codes >> (4 * j)) & 15ull) == static_cast<u64>(c)) mask |= 1u << j;
+            const unsigned bal = __ballot_sync(0xffffffffu, mask != 0);
+            const int at = __shfl_sync(0xffffffffu, count, c) + __popc(bal & ((1u << lane) - 1u));
+            if (mask) mine[c * cap + at] = static_cast<uint32_t>(b) << 8 | mask;
+            if (lane == c) count += __popc(bal);
         }
     }
-    __syncthreads();
-    if (threadIdx.x < kStageCodes) unit_count[blockIdx.x * kStageCodes + threadIdx.x] = s_n[threadIdx.x];
+    if (lane < kStageCodes) unit_count[ch * kStageCodes + lane] = count;
 }
 
-// Rows of the table: row_base[n] + k is sample k of node n. Pass 1 takes them frame by frame and within a
-// frame in Morton (Z) order of (y, x), so that the rows a CTA takes lie in a compact patch; rows without a
-// checked reciprocal come last, in the same order.
+// Rows of the table: row_base[n] + k is sample k of node n; with `both`, row rows + r is the flipped response of
+// row r's sample, used where that sample is evaluated both ways (flip 2). Pass 1 takes them frame by frame and
+// within a frame in Morton (Z) order of (y, x), so that the rows a CTA takes lie in a compact patch; rows without
+// a checked reciprocal come after the others in the same order, unused rows last.
 __global__ void stage_rows_kernel(const NodeDesc* __restrict__ nodes, const long long* __restrict__ row_base, int M,
-                                  long long rows, const Sample* __restrict__ samples, const int* __restrict__ reach,
-                                  int padded, int frame_bits, int* __restrict__ row_pos, uint8_t* __restrict__ row_label,
-                                  u64* __restrict__ key, int* __restrict__ row_ids, float* __restrict__ row_inv,
-                                  int* __restrict__ flip_both) {
+                                  long long rows, int both, const Sample* __restrict__ samples,
+                                  const int* __restrict__ reach, int padded, int morton_bits, int frame_bits,
+                                  int* __restrict__ row_pos, uint8_t* __restrict__ row_label,
+                                  uint8_t* __restrict__ row_both, u64* __restrict__ key, int* __restrict__ row_ids,
+                                  float* __restrict__ row_inv) {
     const long long r = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (r >= rows) return;
     int lo = 0, hi = M - 1;   // the last node n with row_base[n] <= r
@@ -138,45 +129,59 @@ __global__ void stage_rows_kernel(const NodeDesc* __restrict__ nodes, const long
     row_pos[r] = static_cast<int>(p);
     row_label[r] = s.label;
     row_ids[r] = static_cast<int>(r);
-    if (s.flip == 2) *flip_both = 1;
     float inv = 1.0f;   // an invalid depth scales nothing
     if (s.depth > 0.0f)
         inv = s.depth >= 1e-3f && s.depth <= 1e6f ? checked_reciprocal(s.depth, *reach) : 0.0f;   // |v / d| < 2^18
     if (!padded) inv = 0.0f;
     row_inv[r] = inv;
-    key[r] = (inv == 0.0f ? 1ull << (kMorton + frame_bits) : 0ull) | static_cast<u64>(s.image) << kMorton |
-             spread_bits(s.y) << 1 | spread_bits(s.x);
+    const int general_bit = morton_bits + frame_bits;
+    const u64 k = (inv == 0.0f ? 1ull << general_bit : 0ull) | static_cast<u64>(s.image) << morton_bits |
+                  spread_bits(s.y) << 1 | spread_bits(s.x);
+    key[r] = k;
+    if (both) {
+        row_both[r] = s.flip == 2 ? 1 : 0;
+        row_ids[rows + r] = static_cast<int>(rows + r);
+        key[rows + r] = s.flip == 2 ? k : 3ull << general_bit;
+    }
 }
 
-// The rows in key order, and where the rows without a checked reciprocal begin.
-__global__ void stage_list_kernel(long long rows, int general_bit, const u64* __restrict__ key,
+// The rows in key order; ends[0]: the first without a checked reciprocal, ends[1]: the first unused one.
+__global__ void stage_list_kernel(long long rows, long long list_rows, int general_bit, const u64* __restrict__ key,
                                   const int* __restrict__ order, const int* __restrict__ row_pos,
                                   const Sample* __restrict__ samples, const float* __restrict__ row_inv,
-                                  int* __restrict__ general_begin, StageSample* __restrict__ out) {
+                                  int* __restrict__ ends, StageSample* __restrict__ out) {
     const long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (k >= rows) return;
+    if (k >= list_rows) return;
     const int row = order[k];
-    const Sample s = samples[row_pos[row]];
+    const int from = row < rows ? row : row - static_cast<int>(rows);
+    const Sample s = samples[row_pos[from]];
     StageSample o;
     o.x = s.x;
     o.y = s.y;
     o.image = s.image;
-    o.row = static_cast<uint32_t>(row) | (s.flip == 1 ? 0x80000000u : 0u);
-    o.inv_d = s.depth > 0.0f ? row_inv[row] : 0.0f;
+    o.row = static_cast<uint32_t>(row) | (s.flip == 1 || row >= rows ? 0x80000000u : 0u);
+    o.inv_d = s.depth > 0.0f ? row_inv[from] : 0.0f;
     out[k] = o;
-    const bool general = key[k] >> general_bit;
-    if (general && (k == 0 || !(key[k - 1] >> general_bit))) *general_begin = static_cast<int>(k);
-    if (!general && k == rows - 1) *general_begin = static_cast<int>(rows);
+    // 0: gathered, 1: general, 3: unused; the first position of what follows each
+    const int kind = static_cast<int>(key[k] >> general_bit);
+    const int before = k > 0 ? static_cast<int>(key[k - 1] >> general_bit) : 0;
+    if (kind >= 1 && (k == 0 || before < 1)) ends[0] = static_cast<int>(k);
+    if (kind >= 3 && (k == 0 || before < 3)) ends[1] = static_cast<int>(k);
+    if (k == list_rows - 1) {
+        if (kind < 1) ends[0] = static_cast<int>(list_rows);
+        if (kind < 3) ends[1] = static_cast<int>(list_rows);
+    }
 }
 
 struct StageArgs {
     DsView ds;
     const Sample* samples;    // the level's samples
     const int* row_pos;
-    long long rows;
+    long long rows;           // of the table
+    long long sample_rows;    // rows past these hold flipped responses
     const StageSample* list;
     const int* order;
-    const int* general_begin;
+    const int* ends;          // list positions: first row without a checked reciprocal, first unused row
     const FeatParams* packs;
     const float* sorted_thr;  // [F][T]
     const float* feature_rows;
@@ -266,7 +271,7 @@ stage_gather_kernel(const __grid_constant__ StageArgs a) {
     int n_units = 0;
     for (int c = 0; c < kStageCodes - 1; c++) n_units += a.unit_count[c];
     const int tiles = (n_units + kUnits - 1) / kUnits;
-    const long long end = *a.general_begin;
+    const long long end = a.ends[0];
     const long long items = (end + kRows - 1) / kRows * a.parts;
     for (long long item = blockIdx.x; item < items; item += gridDim.x) {
         const long long blk = item / a.parts;
@@ -369,9 +374,9 @@ stage_general_kernel(const __grid_constant__ StageArgs a) {
         const int code_a = seg == 0 ? 0 : kStageCodes - 1, code_b = seg == 0 ? kStageCodes - 1 : kStageCodes;
         int n_units = 0;
         for (int c = code_a; c < code_b; c++) n_units += a.unit_count[c];
-        const long long begin = seg == 0 ? *a.general_begin : 0;
+        const long long begin = seg == 0 ? a.ends[0] : 0, end = a.ends[1];
         const int tiles = (n_units + kUnits - 1) / kUnits;
-        const long long items = (a.rows - begin + 255) / 256 * tiles;
+        const long long items = (end - begin + 255) / 256 * tiles;
         for (long long q = blockIdx.x; q < items; q += gridDim.x) {
             const long long blk = q / tiles;
             const int j = static_cast<int>(q - blk * tiles);
@@ -394,11 +399,12 @@ stage_general_kernel(const __grid_constant__ StageArgs a) {
             }
             __syncthreads();
             const long long k = begin + blk * 256 + threadIdx.x;
-            if (k >= a.rows) continue;
+            if (k >= end) continue;
             const int row = a.order[k];
-            const Sample smp = a.samples[a.row_pos[row]];
+            const int from = row < a.sample_rows ? row : row - static_cast<int>(a.sample_rows);
+            const Sample smp = a.samples[a.row_pos[from]];
             const EvalPixel px = make_eval_pixel(a.ds, smp);
-            const bool flip = smp.flip == 1;
+            const bool flip = smp.flip == 1 || row >= a.sample_rows;
             for (int u = 0; u < nu; u++) {
                 const uint32_t unit = s_unit[u];
                 const uint32_t mask = unit & 255u;
@@ -442,57 +448,55 @@ void launch_general(cf_context* ctx, const char* name, const StageArgs& a) {
 
 }  // namespace
 
+// The padded threshold rows serve T <= 63, the float offsets frames of up to 2^24 bytes of colour integrals
+// (1280x960: 14.7 MB); otherwise every row takes the general kernel.
+bool BinStager::gathers(const DsView& ds, int T) { return T <= kMaxPaddedT && ds.plane <= kMaxBoxPlane; }
+
 void BinStager::prepare(cf_context* ctx, const DsView& ds, const Sample* samples, const NodeDesc* nodes_dev, int M,
-                        const long long* row_base_dev, long long rows, const LevelFeatures& lf, int chunk,
-                        int n_chunks, uint8_t* row_label, int* flip_both) {
-    rows_ = rows;
+                        const long long* row_base_dev, long long rows, bool both, const LevelFeatures& lf, int chunk,
+                        int n_chunks, uint8_t* row_label, uint8_t* row_both) {
+    sample_rows_ = rows;
+    list_rows_ = both ? 2 * rows : rows;
     chunk_ = chunk;
     cap_ = (chunk + kStageUnit - 1) / kStageUnit;
-    // the padded threshold rows serve T <= 63, the float offsets frames of up to 2^24 bytes of depth integral
-    // (1280x960: 9.8 MB); otherwise every row takes the general kernel
-    padded_ = lf.T <= kMaxPaddedT && ds.plane <= kMaxBoxPlane;
-    int frame_bits = 1;
+    padded_ = gathers(ds, lf.T);
+    int frame_bits = 1, pixel_bits = 1;
     while ((1ll << frame_bits) < ds.n) frame_bits++;
+    while ((1 << pixel_bits) < std::max(ds.width, ds.height)) pixel_bits++;
+    const int general_bit = 2 * pixel_bits + frame_bits;
     cudaStream_t st = ctx->stream;
     reach_.reserve(1);
-    CF_CUDA_CHECK(cudaMemsetAsync(reach_.get(), 0, sizeof(int), st));
-    launch(ctx, "stage_plan", dim3(std::min(64, (lf.F + 255) / 256)), dim3(256), 0, stage_reach_kernel, lf.F, lf.packs.get(),
-           reach_.get());
-    if (padded_) {
-        const int row = feature_row(lf.T);
-        const long long n = (lf.F + kStageUnit - 1ll) / kStageUnit * kStageUnit * row;
-        rows_f_.reserve(n);
-        launch(ctx, "stage_plan", dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, stage_feature_rows_kernel,
-               lf.F, lf.T, row, lf.packs.get(), lf.sorted_thr.get(), rows_f_.get());
-    }
     units_.reserve(static_cast<size_t>(n_chunks) * kStageCodes * cap_);
     unit_count_.reserve(static_cast<size_t>(n_chunks) * kStageCodes);
-    launch(ctx, "stage_plan", dim3(n_chunks), dim3(32), 0, stage_units_kernel, lf.F, chunk, cap_, lf.packs.get(),
-           units_.get(), unit_count_.get());
+    const int row = padded_ ? feature_row(lf.T) : 0;
+    const long long n = (lf.F + kStageUnit - 1ll) / kStageUnit * kStageUnit * std::max(row, kRowParams);
+    if (padded_) rows_f_.reserve(n);
+    const int row_blocks = static_cast<int>((n + 255) / 256);
+    CF_CUDA_CHECK(cudaMemsetAsync(reach_.get(), 0, sizeof(int), st));
+    launch(ctx, "stage_plan", dim3(row_blocks + n_chunks), dim3(256), 0, stage_plan_kernel, lf.F, lf.T, row, row_blocks,
+           chunk, cap_, lf.packs.get(), lf.sorted_thr.get(), rows_f_.get(), reach_.get(), units_.get(),
+           unit_count_.get());
     row_pos_.reserve(rows);
-    row_ids_.reserve(rows);
     row_inv_.reserve(rows);
-    key_.reserve(rows);
-    key_sorted_.reserve(rows);
-    order_.reserve(rows);
-    list_.reserve(rows);
-    general_begin_.reserve(1);
-    CF_CUDA_CHECK(cudaMemsetAsync(flip_both, 0, sizeof(int), st));
-    const dim3 grid(static_cast<unsigned>((rows + 255) / 256));
-    launch(ctx, "stage_rows", grid, dim3(256), 0, stage_rows_kernel, nodes_dev, row_base_dev, M, rows, samples,
-           static_cast<const int*>(reach_.get()), padded_ ? 1 : 0, frame_bits, row_pos_.get(), row_label, key_.get(),
-           row_ids_.get(), row_inv_.get(), flip_both);
-    const int general_bit = kMorton + frame_bits;
+    row_ids_.reserve(list_rows_);
+    key_.reserve(list_rows_);
+    key_sorted_.reserve(list_rows_);
+    order_.reserve(list_rows_);
+    list_.reserve(list_rows_);
+    ends_.reserve(2);
+    launch(ctx, "stage_rows", dim3(static_cast<unsigned>((rows + 255) / 256)), dim3(256), 0, stage_rows_kernel, nodes_dev,
+           row_base_dev, M, rows, both ? 1 : 0, samples, static_cast<const int*>(reach_.get()), padded_ ? 1 : 0,
+           2 * pixel_bits, frame_bits, row_pos_.get(), row_label, row_both, key_.get(), row_ids_.get(), row_inv_.get());
+    const int end_bit = general_bit + (both ? 2 : 1);
     size_t temp = 0;
     CF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, temp, key_.get(), key_sorted_.get(), row_ids_.get(),
-                                                  order_.get(), static_cast<int>(rows), 0, general_bit + 1, st));
+                                                  order_.get(), static_cast<int>(list_rows_), 0, end_bit, st));
     sort_temp_.reserve(temp);
     CF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(sort_temp_.get(), temp, key_.get(), key_sorted_.get(),
-                                                  row_ids_.get(), order_.get(), static_cast<int>(rows), 0,
-                                                  general_bit + 1, st));
-    launch(ctx, "stage_rows", grid, dim3(256), 0, stage_list_kernel, rows, general_bit,
-           static_cast<const u64*>(key_sorted_.get()), order_.get(), row_pos_.get(), samples, row_inv_.get(),
-           general_begin_.get(), list_.get());
+                                                  row_ids_.get(), order_.get(), static_cast<int>(list_rows_), 0, end_bit, st));
+    launch(ctx, "stage_rows", dim3(static_cast<unsigned>((list_rows_ + 255) / 256)), dim3(256), 0, stage_list_kernel, rows,
+           list_rows_, general_bit, static_cast<const u64*>(key_sorted_.get()), order_.get(), row_pos_.get(), samples,
+           row_inv_.get(), ends_.get(), list_.get());
 }
 
 void BinStager::run(cf_context* ctx, const DsView& ds, const Sample* samples, const LevelFeatures& lf, int c,
@@ -501,10 +505,11 @@ void BinStager::run(cf_context* ctx, const DsView& ds, const Sample* samples, co
     a.ds = ds;
     a.samples = samples;
     a.row_pos = row_pos_.get();
-    a.rows = rows_;
+    a.rows = list_rows_;
+    a.sample_rows = sample_rows_;
     a.list = list_.get();
     a.order = order_.get();
-    a.general_begin = general_begin_.get();
+    a.ends = ends_.get();
     a.packs = lf.packs.get();
     a.sorted_thr = lf.sorted_thr.get();
     a.feature_rows = rows_f_.get();
@@ -521,7 +526,7 @@ void BinStager::run(cf_context* ctx, const DsView& ds, const Sample* samples, co
         const size_t smem = sizeof(float) * kTileFeatures * feature_row(lf.T);
         set_smem(kernel, smem, kCtasPerSm);
         // few rows: their features in parts, for about eight work items per resident CTA
-        const long long blocks = (rows_ + kRows - 1) / kRows, slots = static_cast<long long>(ctx->num_sms) * kCtasPerSm;
+        const long long blocks = (list_rows_ + kRows - 1) / kRows, slots = static_cast<long long>(ctx->num_sms) * kCtasPerSm;
         const int tiles = (a.n_feat + kTileFeatures - 1) / kTileFeatures;
         a.parts = static_cast<int>(std::max<long long>(1, std::min<long long>(tiles, 8 * slots / blocks)));
         launch(ctx, "stage_bins", dim3(static_cast<unsigned>(std::min(slots, blocks * a.parts))), dim3(kThreads), smem,

@@ -26,23 +26,26 @@ struct __align__(16) StageSample {
 
 class BinStager {
 public:
+    // Whether the gather kernel serves such frames and thresholds.
+    static bool gathers(const DsView& ds, int T);
     // Orders the level's rows (row_base[n] + k is sample k of node n) and lays out the candidates of its
-    // n_chunks feature chunks of `chunk` features.
+    // n_chunks feature chunks of `chunk` features. With `both` the table has twice the rows: row rows + r is the
+    // flipped response of row r where row_both[r] (its sample has flip 2).
     void prepare(cf_context* ctx, const DsView& ds, const Sample* samples, const NodeDesc* nodes_dev, int M,
-                 const long long* row_base_dev, long long rows, const LevelFeatures& lf, int chunk, int n_chunks,
-                 uint8_t* row_label, int* flip_both);
-    // The bins of chunk c: feature f of the chunk and row r at out[((f / 32) * rows + r) * 32 + f % 32].
+                 const long long* row_base_dev, long long rows, bool both, const LevelFeatures& lf, int chunk, int n_chunks,
+                 uint8_t* row_label, uint8_t* row_both);
+    // The bins of chunk c: feature f of the chunk and table row r at out[((f / 32) * table rows + r) * 32 + f % 32].
     void run(cf_context* ctx, const DsView& ds, const Sample* samples, const LevelFeatures& lf, int c, uint8_t* out);
 
 private:
-    long long rows_ = 0;
+    long long sample_rows_ = 0, list_rows_ = 0;
     int chunk_ = 0, cap_ = 0;
     bool padded_ = false;          // the level's thresholds and frames suit the gather kernel
     DevArray<unsigned long long> key_, key_sorted_;
     DevArray<int> row_pos_, row_ids_, order_;
     DevArray<float> row_inv_;      // [rows] checked reciprocal of each row's depth, 0 if there is none
     DevArray<StageSample> list_;   // [rows] in pass-1 order
-    DevArray<int> general_begin_;  // first list position without a checked reciprocal
+    DevArray<int> ends_;           // list positions: first without a checked reciprocal, first unused
     DevArray<float> rows_f_;       // [F][row] scaled parameters and padded thresholds
     DevArray<uint32_t> units_;     // [chunks][codes][cap] first feature / 8 and the mask of its features
     DevArray<int> unit_count_;     // [chunks][codes]

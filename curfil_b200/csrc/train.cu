@@ -48,17 +48,19 @@ void validate_samples(const cf_dataset* ds, const cf_sample* s, long long n, int
 // [offsets[m], offsets[m + 1]) (a flip-2 sample counts twice). Each thread takes a contiguous range of
 // samples: nodes inside its range are its own rows of `hist`, the (at most two) nodes its range shares
 // with its neighbours are counted in private rows and added afterwards. On invalid input the error is
-// that of the first invalid sample, as validate_samples reports it.
-void scan_samples(const cf_dataset* ds, const cf_sample* s, long long n, int C, const int64_t* offsets, int M,
+// that of the first invalid sample, as validate_samples reports it. With `hist`, returns whether a sample has
+// flip 2.
+bool scan_samples(const cf_dataset* ds, const cf_sample* s, long long n, int C, const int64_t* offsets, int M,
                   uint32_t* hist) {
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     const int T = static_cast<int>(std::max<long long>(1, std::min<long long>(std::min<unsigned>(hw, 16u), n >> 18)));
     if (T == 1 && !hist) {
         validate_samples(ds, s, n, C);
-        return;
+        return false;
     }
     struct Part {
         long long a = 0, b = 0, bad = -1;
+        bool both = false;
         int first = 0, last = 0;
         std::vector<uint32_t> head, tail;
     };
@@ -82,6 +84,7 @@ void scan_samples(const cf_dataset* ds, const cf_sample* s, long long n, int C, 
             if (!hist) continue;
             while (offsets[node + 1] <= i) node++;
             const uint32_t add = x.flip == 2 ? 2u : 1u;
+            p.both |= x.flip == 2;
             if (node == p.first) p.head[x.label] += add;
             else if (node == p.last) p.tail[x.label] += add;
             else hist[static_cast<size_t>(node) * C + x.label] += add;
@@ -97,13 +100,16 @@ void scan_samples(const cf_dataset* ds, const cf_sample* s, long long n, int C, 
     for (std::thread& th : pool) th.join();
     for (const Part& p : parts)   // in sample order: the first invalid sample's error
         if (p.bad >= 0) check_sample(ds, s[p.bad], p.bad, C);
-    if (!hist) return;
+    bool both = false;
+    if (!hist) return both;
     for (const Part& p : parts) {
         if (p.a >= p.b) continue;
+        both |= p.both;
         for (int c = 0; c < C; c++) hist[static_cast<size_t>(p.first) * C + c] += p.head[c];
         if (p.last != p.first)
             for (int c = 0; c < C; c++) hist[static_cast<size_t>(p.last) * C + c] += p.tail[c];
     }
+    return both;
 }
 
 void validate_thresholds(const float* thr, long long n) {
@@ -120,6 +126,7 @@ void validate_thresholds(const float* thr, long long n) {
 struct cf_level_snapshot {
     cf_dataset* ds = nullptr;
     int level = 0, M = 0, C = 0, tree_next = 0;
+    bool may_flip_both = false;           // the training started from samples with flip 2
     long long n = 0;
     uint32_t seed = 0;
     cf_train_config cfg{};
@@ -228,7 +235,7 @@ public:
             counts.resize(M);
             for (int i = 0; i < M; i++) counts[i] = h_nodes[i].count;
             if (captured_ && std::find(capture_.begin(), capture_.end(), level) != capture_.end())
-                captured_->push_back(snapshot(cur, level, M, n, seed, tree_next, counts, h_nodes));
+                captured_->push_back(snapshot(cur, level, M, n, seed, tree_next, any_both, counts, h_nodes));
             cudaEvent_t le0, le1;
             CF_CUDA_CHECK(cudaEventCreate(&le0));
             CF_CUDA_CHECK(cudaEventCreate(&le1));
@@ -243,7 +250,7 @@ public:
                                          static_cast<int>(cfg_.max_samples_per_batch), splits_.get() + i, nullptr);
             } else {
                 eval_.evaluate(ctx, ds, samples_[cur].get(), nodes_[cur].get(), hist_[cur].get(), M, counts, C_, lf_,
-                               splits_.get());
+                               splits_.get(), any_both);
             }
             CF_CUDA_CHECK(cudaEventRecord(le1, st));
             evals += eval_.shard.world > 1 ? eval_.last_local_evals : n * F;
@@ -353,7 +360,7 @@ public:
                                      static_cast<int>(cfg_.max_samples_per_batch), splits_.get() + i, nullptr);
         } else {
             eval_.evaluate(ctx, ds, s->samples.get(), s->nodes.get(), s->hist.get(), M, s->counts, C_, lf_,
-                           splits_.get());
+                           splits_.get(), s->may_flip_both);
         }
         const bool scatter = s->level + 1 < cfg_.max_depth;
         RouteResult rr = route_level(ctx, ds, s->samples.get(), s->snode.get(), n, s->nodes.get(), M, splits_.get(), lf_,
@@ -384,7 +391,7 @@ public:
     } host_;
 
 private:
-    cf_level_snapshot* snapshot(int cur, int level, int M, long long n, uint32_t seed, int tree_next,
+    cf_level_snapshot* snapshot(int cur, int level, int M, long long n, uint32_t seed, int tree_next, bool may_flip_both,
                                 const std::vector<int>& counts, const std::vector<NodeDesc>& h_nodes) {
         std::unique_ptr<cf_level_snapshot> s(new cf_level_snapshot());
         s->ds = ds_;
@@ -394,6 +401,7 @@ private:
         s->n = n;
         s->seed = seed;
         s->tree_next = tree_next;
+        s->may_flip_both = may_flip_both;
         s->cfg = cfg_;
         s->counts = counts;
         s->offsets.resize(M + 1);
@@ -647,7 +655,7 @@ void evaluate_level_host(cf_dataset* ds, int num_nodes, const int64_t* node_offs
         // the copy before they pass
         upload_samples(ctx, hc.samples, samples, n);
         std::vector<uint32_t> hist(static_cast<size_t>(num_nodes) * num_classes, 0);
-        scan_samples(ds, samples, n, num_classes, node_offsets, num_nodes, hist.data());
+        const bool any_both = scan_samples(ds, samples, n, num_classes, node_offsets, num_nodes, hist.data());
         validate_thresholds(thresholds, static_cast<long long>(num_features) * num_thresholds);
         DevArray<NodeDesc>& d_nodes = hc.nodes;
         DevArray<uint32_t>& d_hist = hc.hist;
@@ -674,7 +682,7 @@ void evaluate_level_host(cf_dataset* ds, int num_nodes, const int64_t* node_offs
             CF_CUDA_CHECK(cudaMemsetAsync(d_left.get(), 0, sizeof(uint32_t) * n_left, ctx->stream));
         }
         ev.evaluate(ctx, view_of(ds), hc.samples.get(), d_nodes.get(), d_hist.get(), num_nodes, counts, num_classes,
-                    lf, d_best.get(), left_counts ? d_left.get() : nullptr);
+                    lf, d_best.get(), any_both, left_counts ? d_left.get() : nullptr);
         CF_CUDA_CHECK(cudaMemcpyAsync(best, d_best.get(), sizeof(cf_split) * num_nodes, cudaMemcpyDeviceToHost,
                                       ctx->stream));
         if (left_counts)

@@ -126,13 +126,15 @@ typedef struct cf_eval_tuning {
                                     much work, whichever is fewer. Many items per node keep many CTAs on
                                     the same samples at once (their gathers share L2), but small items
                                     pay their setup more often */
-    int32_t stage_bins;          /* 1 (default): when the integral images exceed the L2 cache, every level
-                                    is searched in two passes: the threshold bins of every (sample,
-                                    feature) are computed in frame order (the gathers of one frame's
-                                    samples share L2) into a byte table, then histogrammed node by node
-                                    (huge nodes in sample slices). 0: never; 2: always (T <= 255) */
-    int32_t stage_max_mb;        /* device memory of the staged bin table at most, 1..65536 MiB (default 8192);
-                                    a level whose table is larger runs in feature chunks */
+    int32_t stage_bins;          /* 1 (default): when the integral images exceed the L2 cache, and on other levels
+                                    of at least 2^23 (sample, feature) pairs (2^21 with 256 features and 64
+                                    nodes) with T <= 63 and frames of up to 1.39 M pixels, a level is searched
+                                    in two passes: the threshold bins of every (sample, feature) are computed
+                                    in frame order into a byte table, then histogrammed node by node (huge
+                                    nodes in sample slices). 0: never; 2: always (T <= 255) */
+    int32_t stage_max_mb;        /* device memory of the staged bin table at most, 1..65536 MiB (default 8192; twice
+                                    that where samples are evaluated both ways, flip 2); a level whose table is
+                                    larger runs in feature chunks */
     int32_t sample_order;        /* levels searched in one pass: 1 (default) reads a copy of the samples sorted
                                     by (node, frame, Morton code of the pixel) where the integral images
                                     exceed the L2 cache, so a CTA's samples lie in a compact patch and
