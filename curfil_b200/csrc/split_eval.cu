@@ -1243,6 +1243,18 @@ void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* s
             stage = false;   // no room for the second half of the table: one pass
         }
     }
+    if (stage) {
+        // pass 1 of the first chunk needs no work items: it runs while the host lays them out (about 1 ms for the
+        // 12 000 items of a deep level of 500 nodes, a tenth of the level's time)
+        queue_.reserve(n_chunks);
+        CF_CUDA_CHECK(cudaMemsetAsync(queue_.get(), 0, sizeof(int) * n_chunks, ctx->stream));
+        set_row_base(ctx, M, node_counts);
+        row_label_.reserve(rows);
+        if (may_flip_both) row_both_.reserve(rows);
+        stager_.prepare(ctx, ds, samples, nodes_dev, M, row_base_.get(), rows, may_flip_both, lf, stage_chunk, n_chunks,
+                        row_label_.get(), row_both_.get());
+        stager_.run(ctx, ds, samples, lf, 0, stage_.get());
+    }
     // the staged search reads bytes instead of gathering, so it needs no L1: a larger histogram and
     // tiles of up to 32 features, and items of whole 32-feature rows (fewer, larger items: no CTAs
     // need to share a node's gathers)
@@ -1284,14 +1296,16 @@ void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* s
     order_.reserve(n_items);
     item_range_.reserve(M + 1);
     cands_.reserve(n_items);
-    queue_.reserve(1);
     CF_CUDA_CHECK(cudaMemcpyAsync(items_.get(), h_items_.data(), sizeof(EvalItem) * n_items, cudaMemcpyHostToDevice,
                                   ctx->stream));
     CF_CUDA_CHECK(cudaMemcpyAsync(order_.get(), h_local_order_.data(), sizeof(int) * std::max(1, n_local),
                                   cudaMemcpyHostToDevice, ctx->stream));
     CF_CUDA_CHECK(cudaMemcpyAsync(item_range_.get(), h_range_.data(), sizeof(int) * (M + 1), cudaMemcpyHostToDevice,
                                   ctx->stream));
-    CF_CUDA_CHECK(cudaMemsetAsync(queue_.get(), 0, sizeof(int), ctx->stream));
+    if (!stage) {
+        queue_.reserve(1);
+        CF_CUDA_CHECK(cudaMemsetAsync(queue_.get(), 0, sizeof(int), ctx->stream));
+    }
     if (n_groups > 0) {
         group_bins_.reserve(static_cast<size_t>(n_groups) * budget);
         group_count_.reserve(n_groups);
@@ -1327,13 +1341,6 @@ void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* s
     launch(ctx, "node_consts", dim3((M + 127) / 128), dim3(128), 0, node_consts_kernel, M, C, node_hist_dev,
            reinterpret_cast<NodeConsts*>(node_consts_.get()));
     if (stage) {
-        queue_.reserve(n_chunks);
-        CF_CUDA_CHECK(cudaMemsetAsync(queue_.get(), 0, sizeof(int) * n_chunks, ctx->stream));
-        set_row_base(ctx, M, node_counts);
-        row_label_.reserve(rows);
-        if (may_flip_both) row_both_.reserve(rows);
-        stager_.prepare(ctx, ds, samples, nodes_dev, M, row_base_.get(), rows, may_flip_both, lf, stage_chunk, n_chunks,
-                        row_label_.get(), row_both_.get());
         args.staged = stage_.get();
         args.staged_rows = table_rows;
         args.row_label = row_label_.get();
@@ -1341,7 +1348,7 @@ void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* s
         args.row_both = may_flip_both ? row_both_.get() : nullptr;
         args.both_rows = rows;
         for (int c = 0; c < n_chunks; c++) {
-            stager_.run(ctx, ds, samples, lf, c, stage_.get());
+            if (c > 0) stager_.run(ctx, ds, samples, lf, c, stage_.get());
             args.staged_f0 = c * stage_chunk;
             args.order = order_.get() + h_chunk_begin_[c];
             args.n_items = h_chunk_begin_[c + 1] - h_chunk_begin_[c];
