@@ -10,10 +10,12 @@
 //     99.9 % of the depths in whole millimetres; rows of other depths take the general kernel). v i + 2^23
 //     rounded toward zero is then one instruction for two values, and corner offsets are computed as floats
 //     whose bits are the integer;
-//   - a CTA keeps 64 neighbouring samples (frame and Morton order) and walks all features of the chunk, so the
-//     patch that its corners lie in stays in L1 (hit rate 87 %, against 51 % for 256 samples x 64 features).
-// 800 000 samples, 4000 features x 32 thresholds (100 frames 640x480): 49.0 ms before, 31.5 ms after; 8 M samples on
-// 1000 frames: 519 ms, then 320 ms.
+//   - an SM keeps 32 neighbouring samples at a time (frame and Morton order), and its 24 warps walk their features
+//     side by side, so the patch that the corners lie in stays in L1: misses cost cycles of the same pipe.
+// 800 000 samples, 4000 features x 32 thresholds (100 frames 640x480, a sample per 38 pixels): 49.0 ms with 256
+// samples x 64 features a CTA, 31.5 ms with two CTAs of 64 samples and a barrier per 128 features, 28.2 ms this way.
+// A tree of 266 600 samples, 2000 x 20 (200 frames, a sample per 230 pixels; hit rate 54 % with the barriers): 145.6 ms,
+// then 103.2 ms over its 19 levels; 8 M samples on 1000 frames: 519, 320 and 294 ms.
 //
 // The bin is the one feature_bin gives, in every case: depth means are compared in float with an error
 // bound and a threshold within it is decided by the exact division; colour sums are exact in double.
@@ -30,10 +32,9 @@ namespace cf {
 
 namespace {
 
-constexpr int kThreads = 512;         // 16 warps: kRows / 32 groups of lanes x 8 unit columns
-constexpr int kCtasPerSm = 2;         // 64 registers; the shared memory left over is L1
-constexpr int kRows = 64;             // samples of a CTA (32: idle lanes of the tag pipe; 128, 256: 2-8 % slower)
-constexpr int kTileFeatures = 128;    // features staged at a time
+constexpr int kThreads = 768;         // 24 warps of 80 registers (512: 2 %, 1024 with 64 registers: 1 % slower)
+constexpr int kRows = 32;             // samples of a CTA, one to a lane (64, or two CTAs of 32: 10-20 % slower)
+constexpr int kStep = 2;              // features of a copy to shared memory (4: more of it, 2 % slower)
 constexpr int kGeneralTile = 16;      // features per work item of the general kernel, which mostly takes few rows:
                                       // 64 kept one CTA 45-90 us on the few rows of a small level
 constexpr int kGeneralCtasPerSm = 3;
@@ -198,6 +199,18 @@ __device__ __forceinline__ uint8_t* bin_place(const StageArgs& a, int g, long lo
     return a.out + (((g >> 5) * a.rows + row) << 5) + (g & 31);
 }
 
+__device__ __forceinline__ void cp_async16(void* shared, const void* global) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(shared))),
+                 "l"(global)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kPending>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
+}
+
 // Thresholds below v of a padded row (32 entries serve T <= 31, 36 T = 32, 64 T <= 63): halving, on a byte
 // offset so that a step is a read, a compare and an addition.
 template <int kRow>
@@ -253,105 +266,134 @@ __device__ __forceinline__ int color_bin(const BoxLane& l, const float* row, con
     return k.in && !isnan(r) ? bin : T;
 }
 
-// One work item = 64 rows of the list x the chunk's features (in `parts` parts where there are few rows). The
-// lanes of a warp keep 32 samples, the CTA's eight unit columns share each group of samples and take the
-// tile's 8-feature units in turn, two features of a unit at a time so that their gathers overlap, and store a
-// unit's bins as one 8-byte word.
+// One work item = 32 rows of the list x the chunk's features (in `parts` parts where there are few rows), its
+// features in units of eight. A warp's lanes keep the 32 samples. The warps of a CTA take the next unit of its items
+// in turn: they stay on the same rows and on neighbouring features, so that their corners share L1, without waiting
+// for one another (with a barrier per 128 features: 17 % slower on 500 features). The rows of the next two features
+// are copied to the warp's own shared memory while two are evaluated, whose gathers overlap; a unit's bins are stored
+// as one 8-byte word.
 template <int kRow>
-__global__ void __launch_bounds__(kThreads, kCtasPerSm)
+__global__ void __launch_bounds__(kThreads, 1)
 stage_gather_kernel(const __grid_constant__ StageArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
-    float* rows = reinterpret_cast<float*>(smem);
-    constexpr int kUnits = kTileFeatures / kStageUnit;
-    constexpr int kGroups = kRows / 32, kColumns = kThreads / kRows;
-    __shared__ uint32_t s_unit[kUnits];
+    __shared__ unsigned s_next;   // units of this CTA's items that are taken
     const int T = a.T;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int column = warp / kGroups;
-    int n_units = 0;
-    for (int c = 0; c < kStageCodes - 1; c++) n_units += a.unit_count[c];
-    const int tiles = (n_units + kUnits - 1) / kUnits;
-    const long long end = a.ends[0];
-    const long long items = (end + kRows - 1) / kRows * a.parts;
-    for (long long item = blockIdx.x; item < items; item += gridDim.x) {
-        const long long blk = item / a.parts;
-        const int part = static_cast<int>(item - blk * a.parts);
-        const long long k = blk * kRows + (warp % kGroups) * 32 + lane;
-        const bool have = k < end;
-        const StageSample s = a.list[have ? k : end - 1];
-        const bool valid = s.inv_d > 0.0f;
-        BoxLane l;
-        const float inv = valid ? s.inv_d : 1.0f;
-        l.pos = pack_f2(static_cast<float>(s.x), static_cast<float>(s.y));
-        l.inv = pack_f2(inv, inv);
-        l.side = pack_f2(s.row >> 31 ? -1.0f : 1.0f, 1.0f);
-        const int row = static_cast<int>(s.row & 0x7FFFFFFFu);
-        const unsigned char* depth = reinterpret_cast<const unsigned char*>(a.ds.depth + s.image * a.ds.plane);
-        const unsigned char* color = reinterpret_cast<const unsigned char*>(a.ds.color + s.image * 3ll * a.ds.plane);
-        FrameView view;
-        view.xmax = static_cast<float>(a.ds.width - 1);
-        view.ymax = static_cast<float>(a.ds.height - 1);
-        const int plane = static_cast<int>(a.ds.plane) * 4;
-        for (int j = tiles * part / a.parts; j < tiles * (part + 1) / a.parts; j++) {
-            const int nu = min(kUnits, n_units - j * kUnits);
-            __syncthreads();   // the previous tile is read
-            if (static_cast<int>(threadIdx.x) < nu) {
-                int v = j * kUnits + threadIdx.x, c = 0;
-                while (v >= a.unit_count[c]) v -= a.unit_count[c++];
-                s_unit[threadIdx.x] = a.units[c * a.cap + v] | static_cast<uint32_t>(c) << 28;
+    float* rows = reinterpret_cast<float*>(smem) + warp * 2 * kStep * kRow;   // two steps of the warp's
+    if (threadIdx.x == 0) s_next = 0;
+    __syncthreads();
+    // lane c: the units of codes 0 .. c
+    int upto = lane < kStageCodes - 1 ? a.unit_count[lane] : 0;
+    for (int o = 1; o < kStageCodes; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+    }
+    const int n_units = __shfl_sync(0xffffffffu, upto, kStageCodes - 2);
+    const unsigned per = (n_units + a.parts - 1) / a.parts;   // units of an item; a last part may hold fewer
+    const int end = a.ends[0];
+    const int items = static_cast<int>((end + kRows - 1ll) / kRows) * a.parts;
+    if (n_units == 0) return;
+
+    BoxLane l;
+    FrameView view;
+    view.xmax = static_cast<float>(a.ds.width - 1);
+    view.ymax = static_cast<float>(a.ds.height - 1);
+    const int plane = static_cast<int>(a.ds.plane) * 4;
+    const unsigned char *depth = nullptr, *color = nullptr;
+    bool have = false, valid = false;
+    int row = 0, block = -1;
+
+    // the next unit of this CTA's items: its item, and the entry of its list with the code above bit 28
+    auto take = [&](int& item, uint32_t& unit) {
+        for (;;) {
+            unsigned q = 0;
+            if (lane == 0) q = atomicAdd(&s_next, 1u);
+            q = __shfl_sync(0xffffffffu, q, 0);
+            const unsigned turn = q / per;
+            const long long at = blockIdx.x + static_cast<long long>(turn) * gridDim.x;
+            item = at < items ? static_cast<int>(at) : -1;
+            if (item < 0) return;
+            const int u = static_cast<int>(item % a.parts * per + (q - turn * per));
+            if (u >= n_units) continue;
+            const int c = __popc(__ballot_sync(0xffffffffu, lane < kStageCodes - 1 && upto <= u));
+            const int first = __shfl_sync(0xffffffffu, upto, max(c - 1, 0));
+            unit = __ldg(a.units + c * a.cap + u - (c > 0 ? first : 0)) | static_cast<uint32_t>(c) << 28;
+            return;
+        }
+    };
+    auto fetch = [&](uint32_t unit, int step) {
+        const int f0 = a.f_first + static_cast<int>(unit >> 8 & 0xFFFFFu) * kStageUnit + step * kStep;
+        const float* from = a.feature_rows + static_cast<long long>(f0) * kRow;
+        float* to = rows + (step & 1) * kStep * kRow;
+        for (int i = lane; i < kStep * kRow / 4; i += 32) cp_async16(to + 4 * i, from + 4 * i);
+    };
+
+    int next_item;
+    uint32_t next = 0;
+    take(next_item, next);
+    if (next_item >= 0) fetch(next, 0);
+    cp_async_commit();
+    while (next_item >= 0) {
+        const uint32_t unit = next;
+        const int blk = next_item / a.parts;
+        if (blk != block) {
+            block = blk;
+            const long long k = static_cast<long long>(blk) * kRows + lane;
+            have = k < end;
+            const StageSample s = a.list[have ? k : end - 1];
+            valid = s.inv_d > 0.0f;
+            const float inv = valid ? s.inv_d : 1.0f;
+            l.pos = pack_f2(static_cast<float>(s.x), static_cast<float>(s.y));
+            l.inv = pack_f2(inv, inv);
+            l.side = pack_f2(s.row >> 31 ? -1.0f : 1.0f, 1.0f);
+            row = static_cast<int>(s.row & 0x7FFFFFFFu);
+            depth = reinterpret_cast<const unsigned char*>(a.ds.depth + s.image * a.ds.plane);
+            color = reinterpret_cast<const unsigned char*>(a.ds.color + s.image * 3ll * a.ds.plane);
+        }
+        take(next_item, next);
+        const int code = unit >> 28;
+        uint32_t lo = 0, hi = 0;
+#pragma unroll 1
+        for (int step = 0; step < kStageUnit / kStep; step++) {
+            if (step + 1 < kStageUnit / kStep) fetch(unit, step + 1);
+            else if (next_item >= 0) fetch(next, 0);
+            cp_async_commit();
+            cp_async_wait<1>();
+            __syncwarp();
+            const float* r = rows + (step & 1) * kStep * kRow;
+            int b0, b1;
+            if (code == 0) {
+                view.size = __int_as_float(8);
+                view.pitch = __int_as_float(8 * a.ds.width);
+                view.base1 = view.base2 = 0.0f;
+                DepthBoxes x0, x1;
+                bool open0, open1;
+                b0 = depth_bin<kRow>(l, r, depth, view, T, x0, open0);
+                b1 = depth_bin<kRow>(l, r + kRow, depth, view, T, x1, open1);
+                if (open0) b0 = open_bin<kRow>(x0.s1, x0.n1, x0.s2, x0.n2, r + kRowParams);
+                if (open1) b1 = open_bin<kRow>(x1.s1, x1.n1, x1.s2, x1.n2, r + kRow + kRowParams);
+            } else {
+                view.size = __int_as_float(4);
+                view.pitch = __int_as_float(4 * a.ds.width);
+                view.base1 = __int_as_float((code - 1) / 3 * plane);
+                view.base2 = __int_as_float((code - 1) % 3 * plane);
+                b0 = color_bin<kRow>(l, r, color, view, T);
+                b1 = color_bin<kRow>(l, r + kRow, color, view, T);
             }
-            __syncthreads();
-            constexpr int kQuads = kStageUnit * kRow / 4;
-            for (int i = threadIdx.x; i < nu * kQuads; i += kThreads) {
-                const int u = i / kQuads;
-                const int f0 = a.f_first + static_cast<int>(s_unit[u] >> 8 & 0xFFFFFu) * kStageUnit;
-                reinterpret_cast<float4*>(rows)[i] = __ldg(
-                    reinterpret_cast<const float4*>(a.feature_rows + static_cast<long long>(f0) * kRow) + (i - u * kQuads));
-            }
-            __syncthreads();
-            for (int u = column; u < nu; u += kColumns) {
-                const uint32_t unit = s_unit[u];
-                const uint32_t mask = unit & 255u;
-                const int code = unit >> 28;
-                const float* r = rows + u * kStageUnit * kRow;
-                uint32_t lo = 0, hi = 0;
-                if (code == 0) {
-                    view.size = __int_as_float(8);
-                    view.pitch = __int_as_float(8 * a.ds.width);
-                    view.base1 = view.base2 = 0.0f;
-                    for (int i = 0; i < kStageUnit; i += 2, r += 2 * kRow) {
-                        DepthBoxes x0, x1;
-                        bool open0, open1;
-                        int b0 = depth_bin<kRow>(l, r, depth, view, T, x0, open0);
-                        int b1 = depth_bin<kRow>(l, r + kRow, depth, view, T, x1, open1);
-                        if (open0) b0 = open_bin<kRow>(x0.s1, x0.n1, x0.s2, x0.n2, r + kRowParams);
-                        if (open1) b1 = open_bin<kRow>(x1.s1, x1.n1, x1.s2, x1.n2, r + kRow + kRowParams);
-                        lo = __byte_perm(lo, hi, 0x5432);                        // (hi, lo) moves down two bytes
-                        hi = __byte_perm(hi, __byte_perm(b0, b1, 0x0040), 0x5432);
-                    }
-                } else {
-                    view.size = __int_as_float(4);
-                    view.pitch = __int_as_float(4 * a.ds.width);
-                    view.base1 = __int_as_float((code - 1) / 3 * plane);
-                    view.base2 = __int_as_float((code - 1) % 3 * plane);
-                    for (int i = 0; i < kStageUnit; i += 2, r += 2 * kRow) {
-                        const int b0 = color_bin<kRow>(l, r, color, view, T);
-                        const int b1 = color_bin<kRow>(l, r + kRow, color, view, T);
-                        lo = __byte_perm(lo, hi, 0x5432);
-                        hi = __byte_perm(hi, __byte_perm(b0, b1, 0x0040), 0x5432);
-                    }
-                }
-                if (!valid) lo = hi = static_cast<uint32_t>(T) * 0x01010101u;
-                if (have) {
-                    uint8_t* to = bin_place(a, static_cast<int>(unit >> 8 & 0xFFFFFu) * kStageUnit, row);
-                    if (mask == 255u) {
-                        *reinterpret_cast<uint2*>(to) = make_uint2(lo, hi);
-                    } else {
-                        const u64 word = static_cast<u64>(hi) << 32 | lo;
-                        for (int i = 0; i < kStageUnit; i++)
-                            if (mask >> i & 1u) to[i] = static_cast<uint8_t>(word >> (8 * i));
-                    }
-                }
+            lo = __byte_perm(lo, hi, 0x5432);                        // (hi, lo) moves down two bytes
+            hi = __byte_perm(hi, __byte_perm(b0, b1, 0x0040), 0x5432);
+            __syncwarp();   // the step is read: the next copy may overwrite it
+        }
+        if (!valid) lo = hi = static_cast<uint32_t>(T) * 0x01010101u;
+        if (have) {
+            const uint32_t mask = unit & 255u;
+            uint8_t* to = bin_place(a, static_cast<int>(unit >> 8 & 0xFFFFFu) * kStageUnit, row);
+            if (mask == 255u) {
+                *reinterpret_cast<uint2*>(to) = make_uint2(lo, hi);
+            } else {
+                const u64 word = static_cast<u64>(hi) << 32 | lo;
+                for (int i = 0; i < kStageUnit; i++)
+                    if (mask >> i & 1u) to[i] = static_cast<uint8_t>(word >> (8 * i));
             }
         }
     }
@@ -523,12 +565,11 @@ void BinStager::run(cf_context* ctx, const DsView& ds, const Sample* samples, co
     if (padded_) {
         auto kernel = lf.T < 32 ? stage_gather_kernel<kRowParams + 32>
                                 : lf.T == 32 ? stage_gather_kernel<kRowParams + 36> : stage_gather_kernel<kRowParams + 64>;
-        const size_t smem = sizeof(float) * kTileFeatures * feature_row(lf.T);
-        set_smem(kernel, smem, kCtasPerSm);
-        // few rows: their features in parts, for about eight work items per resident CTA
-        const long long blocks = (list_rows_ + kRows - 1) / kRows, slots = static_cast<long long>(ctx->num_sms) * kCtasPerSm;
-        const int tiles = (a.n_feat + kTileFeatures - 1) / kTileFeatures;
-        a.parts = static_cast<int>(std::max<long long>(1, std::min<long long>(tiles, 8 * slots / blocks)));
+        const size_t smem = sizeof(float) * (kThreads / 32) * 2 * kStep * feature_row(lf.T);
+        set_smem(kernel, smem, 1);
+        // few rows: their features in parts of at least 128, for about eight work items per CTA
+        const long long blocks = (list_rows_ + kRows - 1) / kRows, slots = ctx->num_sms;
+        a.parts = static_cast<int>(std::max<long long>(1, std::min<long long>((a.n_feat + 127) / 128, 8 * slots / blocks)));
         launch(ctx, "stage_bins", dim3(static_cast<unsigned>(std::min(slots, blocks * a.parts))), dim3(kThreads), smem,
                kernel, a);
     }
