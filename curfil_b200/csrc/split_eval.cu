@@ -250,7 +250,7 @@ level_eval_kernel(EvalArgs a) {
     __shared__ int s_cp;
     __shared__ double s_total, s_hc;
     __shared__ ScoreConsts s_k;
-    __shared__ float s_wmax[8];
+    __shared__ float s_wmax[8], s_wtop[8];
     __shared__ double s_best;
     __shared__ double s_cs[kMaxCand];
     __shared__ int s_ct[kMaxCand], s_cf[kMaxCand];
@@ -642,7 +642,7 @@ level_eval_kernel(EvalArgs a) {
             // final best, so the candidates and the chosen split are those of scoring every pair.
             {
                 float2* s_bounds = reinterpret_cast<float2*>(s_scores);   // slot i: (lb, ub), then the score
-                float lbmax = 0.0f;
+                float lbmax = 0.0f, ubmax = 0.0f;
                 for (int i = tid; i < nf * T; i += blockDim.x) {
                     const int fl = i / T;
                     const int t = i - fl * T;
@@ -650,14 +650,27 @@ level_eval_kernel(EvalArgs a) {
                     const float2 b = score_bounds([&](int c) { return cum[c * T1]; }, s_counts, cp, sk);
                     s_bounds[i] = b;
                     lbmax = fmaxf(lbmax, b.x);
+                    ubmax = fmaxf(ubmax, b.y);
                 }
-                for (int off = 16; off > 0; off >>= 1) lbmax = fmaxf(lbmax, __shfl_xor_sync(kFull, lbmax, off));
-                if (lane == 0) s_wmax[warp] = lbmax;
+                for (int off = 16; off > 0; off >>= 1) {
+                    lbmax = fmaxf(lbmax, __shfl_xor_sync(kFull, lbmax, off));
+                    ubmax = fmaxf(ubmax, __shfl_xor_sync(kFull, ubmax, off));
+                }
+                if (lane == 0) {
+                    s_wmax[warp] = lbmax;
+                    s_wtop[warp] = ubmax;
+                }
                 if (tid == 0) s_nexact = 0;
                 __syncthreads();
-                float m = s_wmax[0];
-                for (int w = 1; w < static_cast<int>(blockDim.x >> 5); w++) m = fmaxf(m, s_wmax[w]);
+                float m = s_wmax[0], top = s_wtop[0];
+                for (int w = 1; w < static_cast<int>(blockDim.x >> 5); w++) {
+                    m = fmaxf(m, s_wmax[w]);
+                    top = fmaxf(top, s_wtop[w]);
+                }
                 const double floor_s = fmax(static_cast<double>(m), s_best) - 1e-13;
+                // a tile below the item's best so far (nine of ten in an item of many tiles) adds no
+                // candidate: straight to the next one (the values compared are the same for all threads)
+                if (static_cast<double>(top) < floor_s) continue;
                 // pairs reaching the floor: scored where found (fused search: the scoring overlaps the
                 // other warps' gathers) or, reading staged bins, listed and scored after one barrier, a
                 // warp each if there are few (latency) or a thread each (throughput); the rest get -inf
