@@ -700,7 +700,8 @@ class Forest:
 
 class PredictGraph:
     """cf_predict_graph: a fixed batch of raw frames predicted by one CUDA graph replay. `rgb`,
-    `depth`, `labels` (and `probabilities`) are numpy views of the graph's pinned staging buffers."""
+    `depth`, `labels` (and `probabilities`) are numpy views of the graph's pinned staging buffers;
+    a view keeps the graph, and so its buffers, until close()."""
 
     def __init__(self, forest, count, width, height, probabilities=False):
         h = _vp()
@@ -711,13 +712,23 @@ class PredictGraph:
         _check(lib().cf_predict_graph_buffers(h, ctypes.byref(rgb), ctypes.byref(dep), ctypes.byref(pr),
                                               ctypes.byref(lab)))
         n, C = int(count), forest.num_classes
+        self._places = dict(rgb=(rgb.value, ctypes.c_uint8, (n, height, width, 3)),
+                            depth=(dep.value, ctypes.c_uint16, (n, height, width)),
+                            labels=(lab.value, ctypes.c_uint8, (n, height, width)),
+                            probabilities=(pr.value, ctypes.c_float, (n, C, height, width)) if probabilities else None)
 
-        def view(ptr, ctype, shape):
-            return np.ctypeslib.as_array(ctypes.cast(ptr, ctypes.POINTER(ctype)), shape=shape)
-        self.rgb = view(rgb, ctypes.c_uint8, (n, height, width, 3))
-        self.depth = view(dep, ctypes.c_uint16, (n, height, width))
-        self.labels = view(lab, ctypes.c_uint8, (n, height, width))
-        self.probabilities = view(pr, ctypes.c_float, (n, C, height, width)) if probabilities else None
+    def _view(self, name):
+        if self._places[name] is None:
+            return None
+        address, ctype, shape = self._places[name]
+        buffer = (ctype * int(np.prod(shape))).from_address(address)
+        buffer.graph = self   # the array's base holds the graph
+        return np.ctypeslib.as_array(buffer).reshape(shape)
+
+    rgb = property(lambda self: self._view("rgb"))
+    depth = property(lambda self: self._view("depth"))
+    labels = property(lambda self: self._view("labels"))
+    probabilities = property(lambda self: self._view("probabilities"))
 
     def run(self):
         _check(lib().cf_predict_graph_run(self.handle))
