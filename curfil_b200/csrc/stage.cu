@@ -3,7 +3,7 @@
 // A response reads eight corners of the sample's integral images, and the lanes of a corner load (one sample
 // each) fall in as many 128-byte lines, so a load of 32 lanes takes 8 cycles of the L1 tag pipe however its
 // data lies: 64 of them per 32 evaluations, 80 with the parameters and the threshold search. That pipe is
-// what bounds the pass (82 % of its peak); the kernel is laid out to need little else:
+// what bounds the pass (75 % of its peak, issue 55 %); the kernel is laid out to need little else:
 //   - 170 instructions per 32 evaluations (feature_bin of eval_fast.cuh: 311). Depth scaling is the
 //     reference's trunc(RN(v / d)): every sample brings a float i with floor(v i) = trunc(RN(v / d)) for every
 //     magnitude v that the level's candidates hold, checked value by value (RN(1 / d) or the next float serves
