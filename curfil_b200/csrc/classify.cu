@@ -82,7 +82,8 @@ __device__ __forceinline__ u64 sign_pair(u64 v) { return (v & 0x8000000080000000
 // (sector hit rate 47 -> 71 %), and 20 class sums instead of 40 fit in the registers beside the walk. The
 // kernel is bound by instruction issue (73 %) and the L1 tag pipe (73 %): 41 000 warp instructions for 32
 // pixels of 10 trees, 65 700 before the walk used box_fast.cuh; 64 frames 640x480, 40 classes: 39.0 -> 28.4 ms.
-template <int CMAX, int kPixels, int kSplit>
+// kWide: a frame's byte offsets may pass 2^24, so corners are element indices in integers (wide_corners).
+template <int CMAX, int kPixels, int kSplit, bool kWide>
 __global__ void __launch_bounds__(kPixels * kSplit, CMAX / kSplit <= 32 ? 1024 / (kPixels * kSplit) : 1)
 classify_kernel(const PackedNode* __restrict__ nodes, const int* __restrict__ tree_base, int num_trees, int cache,
                 const float* __restrict__ leaves, int leaf_stride, int C, const FrameDesc* __restrict__ frames,
@@ -123,7 +124,8 @@ classify_kernel(const PackedNode* __restrict__ nodes, const int* __restrict__ tr
     const int mm = inside ? pixel_mm(fr.depth, fr.width, x, y) : 0;
     BoxLane px;
     // an invalid depth goes right at every node: the pixel is put outside the frame
-    const float inv_d = mm > 0 && mm < kDepths && plane <= kMaxBoxPlane ? __ldg(inv_mm + mm) : 0.0f;
+    const bool fits = kWide ? max(fr.width, fr.height) <= kMaxWideSide : plane <= kMaxBoxPlane;
+    const float inv_d = mm > 0 && mm < kDepths && fits ? __ldg(inv_mm + mm) : 0.0f;
     const bool general = mm > 0 && inv_d == 0.0f;
     px.pos = pack_f2(mm > 0 ? static_cast<float>(x) : -1e6f, static_cast<float>(y));
     px.inv = pack_f2(inv_d, inv_d);
@@ -165,18 +167,31 @@ classify_kernel(const PackedNode* __restrict__ nodes, const int* __restrict__ tr
                     const uint32_t off = par[0] ^ 0x80808080u, reg = par[1] ^ 0x80808080u;
                     const u64 o1 = byte_pair(off, 0), o2 = byte_pair(off, 2);
                     const bool color = meta >> 26 & 1u;
-                    view.size = __int_as_float(color ? 4 : 8);
-                    view.pitch = __int_as_float(color ? 4 * fr.width : 8 * fr.width);
-                    view.base1 = __int_as_float(color ? static_cast<int>(meta >> 27 & 3u) * static_cast<int>(plane) * 4 : 0);
-                    view.base2 = __int_as_float(color ? static_cast<int>(meta >> 29 & 3u) * static_cast<int>(plane) * 4 : 0);
-                    const Corners k =
-                        corners(px, o1, o2, byte_pair(reg, 0), byte_pair(reg, 2), sign_pair(o1), sign_pair(o2), view);
+                    const u64 r1 = byte_pair(reg, 0), r2 = byte_pair(reg, 2), b1 = sign_pair(o1), b2 = sign_pair(o2);
+                    Corners k;
+                    if (kWide) {
+                        k = wide_corners(px, o1, o2, r1, r2, b1, b2, view.xmax, view.ymax, fr.width);
+                    } else {
+                        view.size = __int_as_float(color ? 4 : 8);
+                        view.pitch = __int_as_float(color ? 4 * fr.width : 8 * fr.width);
+                        view.base1 = __int_as_float(color ? static_cast<int>(meta >> 27 & 3u) * static_cast<int>(plane) * 4 : 0);
+                        view.base2 = __int_as_float(color ? static_cast<int>(meta >> 29 & 3u) * static_cast<int>(plane) * 4 : 0);
+                        k = corners(px, o1, o2, r1, r2, b1, b2, view);
+                    }
                     side = 1;
                     if (color) {
-                        const double r = color_response(k, reinterpret_cast<const unsigned char*>(fr.color));
+                        double r;
+                        if (kWide) {
+                            const float *p1 = fr.color + (meta >> 27 & 3u) * plane, *p2 = fr.color + (meta >> 29 & 3u) * plane;
+                            r = color_response_at(k, [=](int i) { return __ldg(p1 + i); }, [=](int i) { return __ldg(p2 + i); });
+                        } else {
+                            r = color_response(k, reinterpret_cast<const unsigned char*>(fr.color));
+                        }
                         if (k.in && r <= static_cast<double>(nd.threshold)) side = 0;
                     } else {
-                        const DepthBoxes box = depth_boxes(k, reinterpret_cast<const unsigned char*>(fr.depth));
+                        const int2* const depth = fr.depth;
+                        const DepthBoxes box = kWide ? depth_boxes_at(k, [=](int i) { return __ldg(depth + i); })
+                                                     : depth_boxes(k, reinterpret_cast<const unsigned char*>(depth));
                         if (k.in && box.n1 != 0 && box.n2 != 0) {
                             const DepthBounds d = depth_bounds(box);
                             if (d.plain && d.hi < nd.threshold) side = 0;
@@ -327,12 +342,12 @@ __global__ void plain_argmax_kernel(const float* __restrict__ probs, int C, long
     labels[p] = static_cast<uint8_t>(label);
 }
 
-template <int CMAX, int kPixels, int kSplit>
+template <int CMAX, int kPixels, int kSplit, bool kWide = false>
 void launch_classify(cf_context* ctx, cudaStream_t stream, const cf_forest* f, const FrameDesc* frames, int num_frames,
                      int blocks) {
     const size_t smem = sizeof(PackedNode) * f->num_trees * f->cache_per_tree +
                         sizeof(uint32_t) * std::min(f->num_trees, kTreeChunk) * kPixels;
-    auto kernel = classify_kernel<CMAX, kPixels, kSplit>;
+    auto kernel = classify_kernel<CMAX, kPixels, kSplit, kWide>;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CF_CUDA_CHECK(cudaStreamIsCapturing(stream, &cs));
     if (cs == cudaStreamCaptureStatusNone)   // set before capture (an uncaptured pass runs first)
@@ -347,9 +362,16 @@ void launch_classify(cf_context* ctx, cudaStream_t stream, const cf_forest* f, c
 // four 30.0 ms), except one thread for one or three trees, which do not halve, where its class sums fit the
 // registers (3 trees, 13 classes, 4 frames: 479 against 521 us); and four threads and quarter tiles for
 // launches of few tiles, which the longest walk bounds (160x120, 3 trees: 38 against 56 us).
+// Launches with a frame of more than kMaxBoxPlane pixels take the wide form for all their frames: one of 1920x1080,
+// 10 trees, 40 classes, takes 3.30 ms (4.25 ms with the arithmetic of feature_bin inline, 5.85 ms with general_side
+// for every pixel); four of 1280x960, which the float offsets still serve, 7.1 ms.
 template <int CMAX>
 void launch_classify(cf_context* ctx, cudaStream_t stream, const cf_forest* f, const FrameDesc* frames, int num_frames,
-                     int blocks) {
+                     int blocks, bool wide) {
+    if (wide) {
+        launch_classify<CMAX, 128, 2, true>(ctx, stream, f, frames, num_frames, blocks);
+        return;
+    }
     if (blocks < 4 * ctx->num_sms) {
         launch_classify<CMAX, 64, 4>(ctx, stream, f, frames, num_frames, blocks);
         return;
@@ -370,16 +392,17 @@ int classify_blocks_for(int width, int height) {
 }
 
 void classify_frames(cf_context* ctx, const cf_forest* forest, const FrameDesc* frames_dev, int num_frames,
-                     int total_blocks, cudaStream_t stream) {
+                     int total_blocks, long long largest_plane, cudaStream_t stream) {
     if (stream == nullptr) stream = ctx->stream;
+    const bool wide = largest_plane > kMaxBoxPlane;
     const int C = forest->C;
-    if (C <= 8) launch_classify<8>(ctx, stream, forest, frames_dev, num_frames, total_blocks);
-    else if (C <= 16) launch_classify<16>(ctx, stream, forest, frames_dev, num_frames, total_blocks);
-    else if (C <= 32) launch_classify<32>(ctx, stream, forest, frames_dev, num_frames, total_blocks);
-    else if (C <= 40) launch_classify<40>(ctx, stream, forest, frames_dev, num_frames, total_blocks);
-    else if (C <= 64) launch_classify<64>(ctx, stream, forest, frames_dev, num_frames, total_blocks);
-    else if (C <= 128) launch_classify<128>(ctx, stream, forest, frames_dev, num_frames, total_blocks);
-    else launch_classify<256>(ctx, stream, forest, frames_dev, num_frames, total_blocks);
+    if (C <= 8) launch_classify<8>(ctx, stream, forest, frames_dev, num_frames, total_blocks, wide);
+    else if (C <= 16) launch_classify<16>(ctx, stream, forest, frames_dev, num_frames, total_blocks, wide);
+    else if (C <= 32) launch_classify<32>(ctx, stream, forest, frames_dev, num_frames, total_blocks, wide);
+    else if (C <= 40) launch_classify<40>(ctx, stream, forest, frames_dev, num_frames, total_blocks, wide);
+    else if (C <= 64) launch_classify<64>(ctx, stream, forest, frames_dev, num_frames, total_blocks, wide);
+    else if (C <= 128) launch_classify<128>(ctx, stream, forest, frames_dev, num_frames, total_blocks, wide);
+    else launch_classify<256>(ctx, stream, forest, frames_dev, num_frames, total_blocks, wide);
 }
 
 // detail::normalizeHistogram (random_tree.cpp:54-104)
@@ -409,14 +432,16 @@ namespace {
 void predict_frames(cf_forest* f, std::vector<FrameDesc>& frames) {
     cf_context* ctx = f->ctx;
     int blocks = 0;
+    long long largest = 0;
     for (auto& fr : frames) {
+        largest = std::max(largest, static_cast<long long>(fr.width) * fr.height);
         fr.first_block = blocks;
         blocks += classify_blocks_for(fr.width, fr.height);
     }
     f->frames.reserve(frames.size());
     CF_CUDA_CHECK(cudaMemcpyAsync(f->frames.get(), frames.data(), sizeof(FrameDesc) * frames.size(),
                                   cudaMemcpyHostToDevice, ctx->stream));
-    classify_frames(ctx, f, f->frames.get(), static_cast<int>(frames.size()), blocks);
+    classify_frames(ctx, f, f->frames.get(), static_cast<int>(frames.size()), blocks, largest);
 }
 
 }  // namespace
@@ -770,7 +795,7 @@ void enqueue_graph_batch(cf_predict_graph* g, int blocks) {
     CF_CUDA_CHECK(cudaMemcpyAsync(g->depth_mm.get(), g->h_depth.get(), plane * 2 * n, cudaMemcpyHostToDevice, g->stream));
     integrate_frames(ctx, g->rgb.get(), g->depth_mm.get(), g->count, g->width, g->height, g->color.get(), g->dint.get(),
                      g->stream, g->forest->preprocess);
-    classify_frames(ctx, g->forest, g->frames.get(), g->count, blocks, g->stream);
+    classify_frames(ctx, g->forest, g->frames.get(), g->count, blocks, static_cast<long long>(plane), g->stream);
     CF_CUDA_CHECK(cudaMemcpyAsync(g->h_labels.get(), g->labels.get(), plane * n, cudaMemcpyDeviceToHost, g->stream));
     if (g->with_probs)
         CF_CUDA_CHECK(cudaMemcpyAsync(g->h_probs.get(), g->probs.get(), sizeof(float) * plane * g->forest->C * n,

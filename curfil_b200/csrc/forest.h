@@ -32,8 +32,9 @@ struct FrameDesc {
     int pad;
 };
 
+// largest_plane: pixels of the launch's largest frame
 void classify_frames(cf_context* ctx, const cf_forest* forest, const FrameDesc* frames_dev, int num_frames,
-                     int total_blocks, cudaStream_t stream = nullptr);
+                     int total_blocks, long long largest_plane, cudaStream_t stream = nullptr);
 int classify_blocks_for(int width, int height);
 
 }  // namespace cf

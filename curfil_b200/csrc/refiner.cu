@@ -608,7 +608,7 @@ void for_each_frame_features(cf_refiner* r, cf_forest* forest, cf_dataset* ds, i
         fr.first_block = 0;
         fr.pad = 0;
         CF_CUDA_CHECK(cudaMemcpyAsync(r->frames.get(), &fr, sizeof(fr), cudaMemcpyHostToDevice, ctx->stream));
-        classify_frames(ctx, forest, r->frames.get(), 1, classify_blocks_for(W, H));
+        classify_frames(ctx, forest, r->frames.get(), 1, classify_blocks_for(W, H), plane);
         const int radius = std::max(r->cfg.radius1, r->cfg.radius2);
         if (radius <= kBoxMaxRadius) {
             const size_t smem = box_smem(radius);

@@ -308,7 +308,8 @@ struct cf_server {
             integrate_frames(ctx, pl.rgb, pl.depth, 1, batch[i]->W, batch[i]->H, pl.color, pl.integral, slot->stream,
                              forest->preprocess);
         }
-        classify_frames(ctx, forest, slot->frames.get(), static_cast<int>(batch.size()), blocks, slot->stream);
+        classify_frames(ctx, forest, slot->frames.get(), static_cast<int>(batch.size()), blocks, frame_px,
+                        slot->stream);
         for (size_t i = 0; i < batch.size(); i++) {
             Request& r = *batch[i];
             const size_t px = static_cast<size_t>(r.W) * r.H;
