@@ -84,7 +84,7 @@ __device__ __forceinline__ u64 sign_pair(u64 v) { return (v & 0x8000000080000000
 // pixels of 10 trees, 65 700 before the walk used box_fast.cuh; 64 frames 640x480, 40 classes: 39.0 -> 28.4 ms.
 // kWide: a frame's byte offsets may pass 2^24, so corners are element indices in integers (wide_corners).
 template <int CMAX, int kPixels, int kSplit, bool kWide>
-__global__ void __launch_bounds__(kPixels * kSplit, CMAX / kSplit <= 32 ? 1024 / (kPixels * kSplit) : 1)
+__global__ void __launch_bounds__(kPixels * kSplit, CMAX / kSplit <= 40 ? 1024 / (kPixels * kSplit) : 2)
 classify_kernel(const PackedNode* __restrict__ nodes, const int* __restrict__ tree_base, int num_trees, int cache,
                 const float* __restrict__ leaves, int leaf_stride, int C, const FrameDesc* __restrict__ frames,
                 int num_frames, const float* __restrict__ inv_mm) {
@@ -342,7 +342,7 @@ __global__ void plain_argmax_kernel(const float* __restrict__ probs, int C, long
     labels[p] = static_cast<uint8_t>(label);
 }
 
-template <int CMAX, int kPixels, int kSplit, bool kWide = false>
+template <int CMAX, int kPixels, int kSplit, bool kWide>
 void launch_classify(cf_context* ctx, cudaStream_t stream, const cf_forest* f, const FrameDesc* frames, int num_frames,
                      int blocks) {
     const size_t smem = sizeof(PackedNode) * f->num_trees * f->cache_per_tree +
@@ -358,31 +358,43 @@ void launch_classify(cf_context* ctx, cudaStream_t stream, const cf_forest* f, c
               frames, num_frames, f->inv_mm.get());
 }
 
-// Two threads per pixel and half tiles (10 trees, 40 classes, 64 frames 640x480: 28.4 ms; one thread 33.3 ms,
-// four 30.0 ms), except one thread for one or three trees, which do not halve, where its class sums fit the
-// registers (3 trees, 13 classes, 4 frames: 479 against 521 us); and four threads and quarter tiles for
+// Threads per pixel (8 frames 640x480, us, one / two / four threads):
+//   13 classes: 1 tree 385 / 566 / 968, 2 trees 711 / 745 / 1075, 3 trees 1069 / 1174 / 1249, 5 trees 1783 / 1822 / 2010,
+//               7 trees 2523 / 2500 / 2485, 10 trees 3680 / 3506 / 3541
+//   24 classes: 1 tree 441 / 591 / 980, 3 trees 1195 / 1209 / 1313, 5 trees 1979 / 1867 / 2084
+//   40 classes: 1 tree 543 / 661 / 1083, 2 trees 903 / 861 / 1209, 10 trees 4346 / 3689 / 3762
+//  100 classes: 1 tree 2545 / 1518 / 1560, 3 trees 3390 / 2214 / 1974, 10 trees 6307 / 5133 / 4894
+//  256 classes: 1 tree 7012 / 4054 / 3380, 10 trees 17614 / 8997 / 7789
+// So one thread for the few trees over which a second one idles longer than its half of the class sums saves, as long
+// as the sums fit the registers; four threads past 64 classes, where two leave either the sums no registers or the SM
+// too few warps (100 classes, one CTA an SM: 2708 us for one tree, 9708 for ten); two threads in between, and four for
 // launches of few tiles, which the longest walk bounds (160x120, 3 trees: 38 against 56 us).
 // Launches with a frame of more than kMaxBoxPlane pixels take the wide form for all their frames: one of 1920x1080,
 // 10 trees, 40 classes, takes 3.30 ms (4.25 ms with the arithmetic of feature_bin inline, 5.85 ms with general_side
 // for every pixel); four of 1280x960, which the float offsets still serve, 7.1 ms.
-template <int CMAX>
+template <int CMAX, bool kWide>
 void launch_classify(cf_context* ctx, cudaStream_t stream, const cf_forest* f, const FrameDesc* frames, int num_frames,
-                     int blocks, bool wide) {
-    if (wide) {
-        launch_classify<CMAX, 128, 2, true>(ctx, stream, f, frames, num_frames, blocks);
-        return;
-    }
-    if (blocks < 4 * ctx->num_sms) {
-        launch_classify<CMAX, 64, 4>(ctx, stream, f, frames, num_frames, blocks);
-        return;
-    }
-    if constexpr (CMAX <= 32) {
-        if (f->num_trees == 1 || f->num_trees == 3) {
-            launch_classify<CMAX, 128, 1>(ctx, stream, f, frames, num_frames, blocks);
+                     int blocks) {
+    if constexpr (CMAX <= 40) {
+        if (blocks >= 4 * ctx->num_sms && f->num_trees <= (CMAX <= 32 ? 3 : 1)) {
+            launch_classify<CMAX, 128, 1, kWide>(ctx, stream, f, frames, num_frames, blocks);
             return;
         }
     }
-    launch_classify<CMAX, 128, 2>(ctx, stream, f, frames, num_frames, blocks);
+    if constexpr (CMAX <= 64) {
+        if (blocks >= 4 * ctx->num_sms) {
+            launch_classify<CMAX, 128, 2, kWide>(ctx, stream, f, frames, num_frames, blocks);
+            return;
+        }
+    }
+    launch_classify<CMAX, 64, 4, kWide>(ctx, stream, f, frames, num_frames, blocks);
+}
+
+template <int CMAX>
+void launch_classify(cf_context* ctx, cudaStream_t stream, const cf_forest* f, const FrameDesc* frames, int num_frames,
+                     int blocks, bool wide) {
+    if (wide) launch_classify<CMAX, true>(ctx, stream, f, frames, num_frames, blocks);
+    else launch_classify<CMAX, false>(ctx, stream, f, frames, num_frames, blocks);
 }
 
 }  // namespace

@@ -1,5 +1,6 @@
-"""The forms of the prediction kernel (csrc/classify.cu) against the plain form, bit for bit: frames whose byte
-offsets pass 2^24 (element indices in integers), up to sides that take the general responses."""
+"""The forms of the prediction kernel (csrc/classify.cu) against the plain form, bit for bit: one, two and four threads
+a pixel over the class counts of every instance and over more trees than are walked at a time; frames whose byte
+offsets pass 2^24 (element indices in integers), up to sides that take the general responses; padded frames."""
 import numpy as np
 import pytest
 
@@ -102,3 +103,45 @@ def test_long_host_frames_equal_the_plain_form(ctx, w):
     np.testing.assert_array_equal(l1, l2)
     assert len(np.unique(l1[0, 1])) > 1
     forest.close()
+
+
+# 595 tiles of 16 x 16 pixels take the forms of large launches, 35 the four threads of small ones
+@pytest.mark.parametrize("n", [17, 1])
+@pytest.mark.parametrize("trees,C", [(1, 5), (3, 16), (4, 8), (2, 17), (3, 32), (4, 31), (1, 40), (2, 33), (5, 40), (1, 41),
+                                     (3, 64), (1, 65), (3, 128), (2, 129), (1, 256), (32, 7), (33, 13), (33, 40), (65, 3),
+                                     (65, 64), (34, 70)])
+def test_threads_per_pixel_equal_the_plain_form(ctx, n, trees, C):
+    w, h = 97, 71
+    rng = np.random.default_rng(trees * 300 + C)
+    rgb, depth = noisy_frames(rng, n, w, h)
+    ds = cf.Dataset.from_raw(ctx, rgb, depth)
+    assert_equals_plain(ctx, ds, depth, n, w, h, trees, C, seed=trees + C)
+    ds.close()
+
+
+@pytest.mark.parametrize("n", [18, 1])
+def test_padded_frames_equal_the_plain_form(ctx, n):
+    """Corners in the padding hold NaN colours and zero depth integrals: box counts come out zero or negative."""
+    w, h = 96, 72
+    rng = np.random.default_rng(n)
+    rgb, depth = noisy_frames(rng, n, 70, 50)
+    ds = cf.Dataset(ctx, n, w, h)
+    ds.upload_raw_padded(rgb, depth)
+    padded = np.zeros((n, h, w), np.uint16)
+    padded[:, :50, :70] = depth
+    assert_equals_plain(ctx, ds, padded, n, w, h, 5, 13, seed=n)
+    ds.close()
+
+
+def test_depths_past_the_table_equal_the_plain_form(ctx):
+    """Depths above 65.535 m have no checked reciprocal in the forest's table."""
+    n, w, h, C = 17, 97, 71, 13
+    rng = np.random.default_rng(9)
+    rgb, depth = noisy_frames(rng, n, w, h)
+    far = depth.astype(np.int64) * np.where(rng.random(depth.shape) < 0.5, 37, 1)
+    color = np.cumsum(np.cumsum(rgb.transpose(0, 3, 1, 2).astype(np.int64), 3), 2).astype(np.float32)
+    planes = np.stack([np.cumsum(np.cumsum(v, 2), 1) for v in (far, (far > 0).astype(np.int64))], 1).astype(np.int32)
+    ds = cf.Dataset.from_integral(ctx, color, np.ascontiguousarray(planes))
+    assert (far > 65535).mean() > 0.2
+    assert_equals_plain(ctx, ds, depth, n, w, h, 5, C, seed=3)
+    ds.close()
