@@ -720,6 +720,8 @@ class PredictGraph:
     def _view(self, name):
         if self._places[name] is None:
             return None
+        if not self.handle:
+            raise CurfilError(1, "PredictGraph.%s: the graph is closed" % name)
         address, ctype, shape = self._places[name]
         buffer = (ctype * int(np.prod(shape))).from_address(address)
         buffer.graph = self   # the array's base holds the graph
