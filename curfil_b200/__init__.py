@@ -701,7 +701,7 @@ class Forest:
 class PredictGraph:
     """cf_predict_graph: a fixed batch of raw frames predicted by one CUDA graph replay. `rgb`,
     `depth`, `labels` (and `probabilities`) are numpy views of the graph's pinned staging buffers;
-    a view keeps the graph, and so its buffers, until close()."""
+    a view keeps the graph, and so its buffers, until close(). Assigning to one of them copies into the buffer."""
 
     def __init__(self, forest, count, width, height, probabilities=False):
         h = _vp()
@@ -727,10 +727,19 @@ class PredictGraph:
         buffer.graph = self   # the array's base holds the graph
         return np.ctypeslib.as_array(buffer).reshape(shape)
 
-    rgb = property(lambda self: self._view("rgb"))
-    depth = property(lambda self: self._view("depth"))
-    labels = property(lambda self: self._view("labels"))
-    probabilities = property(lambda self: self._view("probabilities"))
+    def _write(self, name, value):
+        view = self._view(name)
+        if view is None:
+            raise AttributeError("PredictGraph.%s: the graph has no such buffer" % name)
+        own = getattr(value, "__array_interface__", None) == view.__array_interface__   # after graph.depth += 1
+        if not own:
+            view[...] = value
+
+    rgb = property(lambda self: self._view("rgb"), lambda self, value: self._write("rgb", value))
+    depth = property(lambda self: self._view("depth"), lambda self, value: self._write("depth", value))
+    labels = property(lambda self: self._view("labels"), lambda self, value: self._write("labels", value))
+    probabilities = property(lambda self: self._view("probabilities"),
+                             lambda self, value: self._write("probabilities", value))
 
     def run(self):
         _check(lib().cf_predict_graph_run(self.handle))
