@@ -44,9 +44,15 @@ def library(monkeypatch):
     return fake
 
 
+@pytest.fixture
+def graph(library):
+    g = cf.PredictGraph(FakeForest(), 2, 6, 5, probabilities=True)
+    yield g
+    g.close()   # while the calls are still replaced
+
+
 @pytest.mark.parametrize("name", ["rgb", "depth", "labels", "probabilities"])
-def test_a_closed_graph_gives_no_views(library, name):
-    graph = cf.PredictGraph(FakeForest(), 2, 6, 5, probabilities=True)
+def test_a_closed_graph_gives_no_views(library, graph, name):
     assert getattr(graph, name).size > 0
     graph.close()
     assert library.destroyed == 1
@@ -57,8 +63,7 @@ def test_a_closed_graph_gives_no_views(library, name):
 
 
 @pytest.mark.parametrize("name", ["rgb", "depth", "labels", "probabilities"])
-def test_assignments_write_the_buffer(library, name):
-    graph = cf.PredictGraph(FakeForest(), 2, 6, 5, probabilities=True)
+def test_assignments_write_the_buffer(library, graph, name):
     buffer = library.memory[["rgb", "depth", "probabilities", "labels"].index(name)]
     view = getattr(graph, name)
     new = np.arange(view.size).reshape(view.shape) % 50
@@ -83,3 +88,4 @@ def test_a_graph_without_probabilities_has_no_buffer_for_them(library):
     assert graph.probabilities is None
     with pytest.raises(AttributeError):
         graph.probabilities = 0
+    graph.close()
