@@ -35,8 +35,13 @@ namespace {
 constexpr int kThreads = 768;         // 24 warps of 80 registers (512: 2 %, 1024 with 64 registers: 1 % slower)
 constexpr int kRows = 32;             // samples of a CTA, one to a lane (64, or two CTAs of 32: 10-20 % slower)
 constexpr int kStep = 2;              // features of a copy to shared memory (4: more of it, 2 % slower)
-constexpr int kGeneralTile = 16;      // features per work item of the general kernel, which mostly takes few rows:
-                                      // 64 kept one CTA 45-90 us on the few rows of a small level
+// Features per work item of the general kernel. Where it takes the few rows without a checked reciprocal, 64 kept one
+// CTA 45-90 us on those of a small level, 16 do not. Where it takes all rows, 32 set up a tile and fetch a sample half
+// as often, once there are kManyItems work items of 32 features per resident CTA. Of 16 / 32 / 64, in ms: 20 000 rows x
+// 300 features 0.261 / 0.363 / 0.537, x 1000 (5.7 items a CTA) 0.572 / 0.578 / 0.963; 50 000 x 500 (7.1) 0.791 / 0.728 /
+// 0.947; 266 600 x 1000 6.25 / 5.88 / 5.90 (100 thresholds); 100 000 x 500 of 1920x1080 1.50 / 1.35 / 1.57.
+constexpr int kSmallTile = 16, kLargeTile = 32;
+constexpr long long kManyItems = 6;
 constexpr int kGeneralCtasPerSm = 3;
 
 // Floats of a feature's row: eight parameters, +-2^23 with the sign of each offset, then the ascending
@@ -400,15 +405,15 @@ stage_gather_kernel(const __grid_constant__ StageArgs a) {
 }
 
 // feature_bin itself: rows without a checked reciprocal with all features, then all rows with the features of
-// other channels. One work item = 256 consecutive rows of the list x up to kGeneralTile features.
-template <int kPad>
+// other channels. One work item = 256 consecutive rows of the list x up to kTile features.
+template <int kPad, int kTile>
 __global__ void __launch_bounds__(256, kGeneralCtasPerSm)
 stage_general_kernel(const __grid_constant__ StageArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     EvalFeat* s_params = reinterpret_cast<EvalFeat*>(smem);
-    float* s_thr = reinterpret_cast<float*>(smem + sizeof(EvalFeat) * kGeneralTile);
-    __shared__ uint32_t s_unit[kGeneralTile / kStageUnit];
-    constexpr int kUnits = kGeneralTile / kStageUnit;
+    float* s_thr = reinterpret_cast<float*>(smem + sizeof(EvalFeat) * kTile);
+    __shared__ uint32_t s_unit[kTile / kStageUnit];
+    constexpr int kUnits = kTile / kStageUnit;
     const int T = a.T;
     const int TP = kPad ? kPad : T;
     const int W = a.ds.width, H = a.ds.height;
@@ -480,12 +485,21 @@ void set_smem(K kernel, size_t smem, int ctas) {
                                        std::min(100, static_cast<int>(std::ceil(100.0 * need / (228.0 * 1024))))));
 }
 
-template <int kPad>
+template <int kPad, int kTile>
 void launch_general(cf_context* ctx, const char* name, const StageArgs& a) {
     const int TP = kPad ? kPad : a.T;
-    const size_t smem = sizeof(EvalFeat) * kGeneralTile + sizeof(float) * kGeneralTile * TP;
-    set_smem(stage_general_kernel<kPad>, smem, kGeneralCtasPerSm);
-    launch(ctx, name, dim3(ctx->num_sms * kGeneralCtasPerSm), dim3(256), smem, stage_general_kernel<kPad>, a);
+    const size_t smem = sizeof(EvalFeat) * kTile + sizeof(float) * kTile * TP;
+    set_smem(stage_general_kernel<kPad, kTile>, smem, kGeneralCtasPerSm);
+    launch(ctx, name, dim3(ctx->num_sms * kGeneralCtasPerSm), dim3(256), smem, stage_general_kernel<kPad, kTile>, a);
+}
+
+template <int kTile>
+void launch_general(cf_context* ctx, const char* name, const StageArgs& a) {
+    switch (padded_row(a.T)) {
+        case 32: launch_general<32, kTile>(ctx, name, a); break;
+        case 64: launch_general<64, kTile>(ctx, name, a); break;
+        default: launch_general<0, kTile>(ctx, name, a); break;
+    }
 }
 
 }  // namespace
@@ -573,12 +587,11 @@ void BinStager::run(cf_context* ctx, const DsView& ds, const Sample* samples, co
         launch(ctx, "stage_bins", dim3(static_cast<unsigned>(std::min(slots, blocks * a.parts))), dim3(kThreads), smem,
                kernel, a);
     }
+    const long long items = (list_rows_ + 255) / 256 * ((a.n_feat + kLargeTile - 1) / kLargeTile);
+    const bool many = !padded_ && items >= kManyItems * ctx->num_sms * kGeneralCtasPerSm;
     const char* name = padded_ ? "stage_general" : "stage_bins";
-    switch (padded_row(lf.T)) {
-        case 32: launch_general<32>(ctx, name, a); break;
-        case 64: launch_general<64>(ctx, name, a); break;
-        default: launch_general<0>(ctx, name, a); break;
-    }
+    if (many) launch_general<kLargeTile>(ctx, name, a);
+    else launch_general<kSmallTile>(ctx, name, a);
 }
 
 }  // namespace cf

@@ -52,3 +52,35 @@ def test_bins_equal_the_fused_search(ctx, T, F, w, h):
     np.testing.assert_array_equal(out[2][1], out[0][1])
     for k in ("score", "feature", "threshold_index", "threshold"):
         np.testing.assert_array_equal(out[2][0][k], out[0][0][k], err_msg=k)
+
+
+@pytest.mark.parametrize("T", [64, 200])
+@pytest.mark.parametrize("rows", [4000, 90000])
+def test_general_bins_of_small_and_large_levels(ctx, T, rows):
+    """Thresholds that the gather kernel does not serve, in levels on both sides of the item count from which the
+    general kernel takes wider tiles (2664 items of 256 rows x 32 features on 148 SMs)."""
+    n, C, F, w, h = 3, 11, 250, 97, 71
+    rgb, depth, labels = H.frames(seed=T, n=n, w=w, h=h, cells=9, classes=C)
+    ds = cf.Dataset.from_raw(ctx, rgb, depth)
+    rng = np.random.default_rng(T + rows)
+    offsets = np.array([0, rows // 7, rows // 7 + 1, rows], np.int64)
+    s = H.random_samples(rng, n, w, h, C, rows, depth=depth)
+    fe = H.random_features(rng, F)
+    r = cf.feature_responses(ds, s[:500], fe)
+    th = np.nan_to_num(r[np.arange(F), rng.integers(0, 500, (T, F))], nan=0.0).astype(np.float32)
+    out = {}
+    try:
+        for stage in (0, 2):
+            ctx.set_tuning(stage_bins=stage)
+            ctx.set_timing(True)
+            ctx.reset_timing()
+            out[stage] = cf.level_left_counts(ds, offsets, s, C, fe, th)
+            assert (ctx.kernel_time("stage_bins")[1] > 0) == (stage == 2)
+            ctx.set_timing(False)
+    finally:
+        ctx.set_timing(False)
+        ctx.set_tuning()
+        ds.close()
+    np.testing.assert_array_equal(out[2][1], out[0][1])
+    for k in ("score", "feature", "threshold_index", "threshold"):
+        np.testing.assert_array_equal(out[2][0][k], out[0][0][k], err_msg=k)
