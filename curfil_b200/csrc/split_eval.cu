@@ -1197,6 +1197,20 @@ void split_items_into_chunks(const std::vector<int>& node_counts, int chunk, int
     for (int c = n_chunks - 1; c >= 0; c--) chunk_begin[c] = std::min(chunk_begin[c], chunk_begin[c + 1]);
 }
 
+std::vector<StageTable> stage_tables(long long rows, int F, long long max_bytes) {
+    const int tiles = (F + kStageTile - 1) / kStageTile;
+    std::vector<StageTable> out;
+    // chunks of whole tiles, as even as possible, then half as large
+    long long most = max_bytes / rows / kStageTile;
+    do {
+        const int m = static_cast<int>(std::max<long long>(1, std::min<long long>(most, tiles)));
+        const int n = (tiles + m - 1) / m, chunk = (tiles + n - 1) / n;
+        out.push_back(StageTable{chunk * kStageTile, (tiles + chunk - 1) / chunk});
+        most = chunk / 2;
+    } while (most >= 1);
+    return out;
+}
+
 void LevelEvaluator::set_row_base(cf_context* ctx, int M, const std::vector<int>& node_counts) {
     h_row_base_.assign(M + 1, 0);
     for (int n = 0; n < M; n++) h_row_base_[n + 1] = h_row_base_[n] + node_counts[n];
@@ -1246,38 +1260,45 @@ void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* s
     // stage_bins = 2 on every level. The bins are bytes (T <= 255)
     long long rows = 0;
     for (int c : node_counts) rows += c;
-    const long long table_rows = may_flip_both ? 2 * rows : rows;
+    const long long table_rows = may_flip_both ? 2 * rows : rows, evals = table_rows * F;
     const size_t frame_bytes = static_cast<size_t>(ds.n) * ds.plane * (3 * sizeof(float) + sizeof(int2));
     bool stage = tuning.stage_bins != 0 && !sharded && T <= 255 && rows > 0 && table_rows < INT_MAX &&
                  (tuning.stage_bins == 2 || frame_bytes > ctx->l2_bytes ||
-                  (BinStager::gathers(ds, T) && (table_rows * F >= kStageMinEvals ||
-                                                 (table_rows * F >= kStageMinEvals / 4 && F >= 256 && M >= 64))));
-    int stage_chunk = 0, n_chunks = 0;
+                  (BinStager::gathers(ds, T) && (evals >= kStageMinEvals ||
+                                                 (evals >= kStageMinEvals / 4 && F >= 256 && M >= 64))));
+    StageTable table{0, 0};
     if (stage) {
-        // feature chunks of whole 32-feature tiles whose table fits stage_max_mb, as even as possible
-        const long long f_pad = (F + kStageTile - 1) / kStageTile * kStageTile;
-        const long long max_bytes = static_cast<long long>(tuning.stage_max_mb) << 20;
-        const long long tiles_max = std::max<long long>(1, max_bytes / rows / kStageTile);
-        n_chunks = static_cast<int>((f_pad / kStageTile + tiles_max - 1) / tiles_max);
-        stage_chunk = static_cast<int>((f_pad / kStageTile + n_chunks - 1) / n_chunks) * kStageTile;
-        n_chunks = (F + stage_chunk - 1) / stage_chunk;
-        try {
-            stage_.reserve(static_cast<size_t>(table_rows) * stage_chunk);
-        } catch (const Error& e) {
-            if (e.code != CF_ERR_OOM || !may_flip_both) throw;
-            stage = false;   // no room for the second half of the table: one pass
+        // everything pass 1 needs is allocated before its first launch: a table that does not fit the memory left
+        // gives way to the next smaller one, and the last to the search in one pass, which needs none of this
+        stage = false;
+        for (const StageTable& t : stage_tables(rows, F, static_cast<long long>(tuning.stage_max_mb) << 20)) {
+            try {
+                queue_.reserve(t.n_chunks);
+                row_base_.reserve(M + 1);
+                row_label_.reserve(rows);
+                if (may_flip_both) row_both_.reserve(rows);
+                stager_.reserve(ctx, ds, rows, may_flip_both, lf, t.chunk, t.n_chunks);
+                stage_.reserve(static_cast<size_t>(table_rows) * t.chunk);
+            } catch (const Error& e) {
+                if (e.code != CF_ERR_OOM) throw;
+                continue;
+            }
+            table = t;
+            stage = true;
+            break;
+        }
+        if (!stage) {
+            stage_.release();
+            stager_.release();
         }
     }
+    const int stage_chunk = table.chunk, n_chunks = table.n_chunks;
     if (stage) {
         // pass 1 of the first chunk needs no work items: it runs while the host lays them out (about 1 ms for the
         // 12 000 items of a deep level of 500 nodes, a tenth of the level's time)
-        queue_.reserve(n_chunks);
         CF_CUDA_CHECK(cudaMemsetAsync(queue_.get(), 0, sizeof(int) * n_chunks, ctx->stream));
         set_row_base(ctx, M, node_counts);
-        row_label_.reserve(rows);
-        if (may_flip_both) row_both_.reserve(rows);
-        stager_.prepare(ctx, ds, samples, nodes_dev, M, row_base_.get(), rows, may_flip_both, lf, stage_chunk, n_chunks,
-                        row_label_.get(), row_both_.get());
+        stager_.prepare(ctx, ds, samples, nodes_dev, M, row_base_.get(), lf, row_label_.get(), row_both_.get());
         stager_.run(ctx, ds, samples, lf, 0, stage_.get());
     }
     // the staged search reads bytes instead of gathering, so it needs no L1: a larger histogram and

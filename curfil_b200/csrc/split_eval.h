@@ -88,6 +88,13 @@ constexpr double kStagedItemsPerSlot = 64.0;  // work items per resident CTA at 
 // one node 241 / 316, in 97 nodes 533 / 467, in 2000 nodes 1503 / 1088; 6 M (100 features) 460 / 481; 9.6 M in one
 // node 492 / 445; 30 M 877 / 773; 120 M in 97 nodes 3288 / 2208.
 constexpr long long kStageMinEvals = 1ll << 23;
+// The table of a staged level: n_chunks chunks of `chunk` features, one in memory at a time.
+struct StageTable {
+    int chunk, n_chunks;
+};
+// The tables a level of `rows` samples may have, in the order in which they are tried until one can be allocated
+// (none: the level is searched in one pass).
+std::vector<StageTable> stage_tables(long long rows, int F, long long max_bytes);
 // Splits every item at the chunk boundaries (multiples of `chunk` features) and orders the items
 // chunk by chunk, largest first within a chunk; chunk_begin[c] is the first order position of chunk c.
 void split_items_into_chunks(const std::vector<int>& node_counts, int chunk, int n_chunks,

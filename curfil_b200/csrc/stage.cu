@@ -49,6 +49,10 @@ constexpr int kGeneralCtasPerSm = 3;
 constexpr int kRowParams = 12;
 constexpr int kMaxPaddedT = 63;
 int feature_row(int T) { return T < 32 ? kRowParams + 32 : T == 32 ? kRowParams + 36 : kRowParams + 64; }
+// Entries of all feature rows, in whole units; where there are no rows (row = 0) their parameters alone are walked.
+long long feature_floats(int F, int row) {
+    return (F + kStageUnit - 1ll) / kStageUnit * kStageUnit * std::max(row, kRowParams);
+}
 
 // Unit lists: depth features, the nine channel pairs, the rest (channels past 2).
 __device__ __forceinline__ int pair_code(const FeatParams& f) {
@@ -508,30 +512,23 @@ void launch_general(cf_context* ctx, const char* name, const StageArgs& a) {
 // (1280x960: 14.7 MB); otherwise every row takes the general kernel.
 bool BinStager::gathers(const DsView& ds, int T) { return T <= kMaxPaddedT && ds.plane <= kMaxBoxPlane; }
 
-void BinStager::prepare(cf_context* ctx, const DsView& ds, const Sample* samples, const NodeDesc* nodes_dev, int M,
-                        const long long* row_base_dev, long long rows, bool both, const LevelFeatures& lf, int chunk,
-                        int n_chunks, uint8_t* row_label, uint8_t* row_both) {
+void BinStager::reserve(cf_context* ctx, const DsView& ds, long long rows, bool both, const LevelFeatures& lf, int chunk,
+                        int n_chunks) {
     sample_rows_ = rows;
     list_rows_ = both ? 2 * rows : rows;
     chunk_ = chunk;
+    n_chunks_ = n_chunks;
     cap_ = (chunk + kStageUnit - 1) / kStageUnit;
     padded_ = gathers(ds, lf.T);
     int frame_bits = 1, pixel_bits = 1;
     while ((1ll << frame_bits) < ds.n) frame_bits++;
     while ((1 << pixel_bits) < std::max(ds.width, ds.height)) pixel_bits++;
-    const int general_bit = 2 * pixel_bits + frame_bits;
-    cudaStream_t st = ctx->stream;
+    morton_bits_ = 2 * pixel_bits;
+    frame_bits_ = frame_bits;
     reach_.reserve(1);
     units_.reserve(static_cast<size_t>(n_chunks) * kStageCodes * cap_);
     unit_count_.reserve(static_cast<size_t>(n_chunks) * kStageCodes);
-    const int row = padded_ ? feature_row(lf.T) : 0;
-    const long long n = (lf.F + kStageUnit - 1ll) / kStageUnit * kStageUnit * std::max(row, kRowParams);
-    if (padded_) rows_f_.reserve(n);
-    const int row_blocks = static_cast<int>((n + 255) / 256);
-    CF_CUDA_CHECK(cudaMemsetAsync(reach_.get(), 0, sizeof(int), st));
-    launch(ctx, "stage_plan", dim3(row_blocks + n_chunks), dim3(256), 0, stage_plan_kernel, lf.F, lf.T, row, row_blocks,
-           chunk, cap_, lf.packs.get(), lf.sorted_thr.get(), rows_f_.get(), reach_.get(), units_.get(),
-           unit_count_.get());
+    if (padded_) rows_f_.reserve(feature_floats(lf.F, feature_row(lf.T)));
     row_pos_.reserve(rows);
     row_inv_.reserve(rows);
     row_ids_.reserve(list_rows_);
@@ -540,19 +537,48 @@ void BinStager::prepare(cf_context* ctx, const DsView& ds, const Sample* samples
     order_.reserve(list_rows_);
     list_.reserve(list_rows_);
     ends_.reserve(2);
+    sort_bytes_ = 0;
+    CF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes_, key_.get(), key_sorted_.get(), row_ids_.get(),
+                                                  order_.get(), static_cast<int>(list_rows_), 0, end_bit(), ctx->stream));
+    sort_temp_.reserve(sort_bytes_);
+}
+
+void BinStager::release() {
+    reach_.release();
+    units_.release();
+    unit_count_.release();
+    rows_f_.release();
+    row_pos_.release();
+    row_inv_.release();
+    row_ids_.release();
+    key_.release();
+    key_sorted_.release();
+    order_.release();
+    list_.release();
+    ends_.release();
+    sort_temp_.release();
+}
+
+void BinStager::prepare(cf_context* ctx, const DsView& ds, const Sample* samples, const NodeDesc* nodes_dev, int M,
+                        const long long* row_base_dev, const LevelFeatures& lf, uint8_t* row_label, uint8_t* row_both) {
+    const long long rows = sample_rows_;
+    const bool both = list_rows_ > rows;
+    cudaStream_t st = ctx->stream;
+    const int row = padded_ ? feature_row(lf.T) : 0;
+    const int row_blocks = static_cast<int>((feature_floats(lf.F, row) + 255) / 256);
+    CF_CUDA_CHECK(cudaMemsetAsync(reach_.get(), 0, sizeof(int), st));
+    launch(ctx, "stage_plan", dim3(row_blocks + n_chunks_), dim3(256), 0, stage_plan_kernel, lf.F, lf.T, row, row_blocks,
+           chunk_, cap_, lf.packs.get(), lf.sorted_thr.get(), rows_f_.get(), reach_.get(), units_.get(),
+           unit_count_.get());
     launch(ctx, "stage_rows", dim3(static_cast<unsigned>((rows + 255) / 256)), dim3(256), 0, stage_rows_kernel, nodes_dev,
            row_base_dev, M, rows, both ? 1 : 0, samples, static_cast<const int*>(reach_.get()), padded_ ? 1 : 0,
-           2 * pixel_bits, frame_bits, row_pos_.get(), row_label, row_both, key_.get(), row_ids_.get(), row_inv_.get());
-    const int end_bit = general_bit + (both ? 2 : 1);
-    size_t temp = 0;
-    CF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, temp, key_.get(), key_sorted_.get(), row_ids_.get(),
-                                                  order_.get(), static_cast<int>(list_rows_), 0, end_bit, st));
-    sort_temp_.reserve(temp);
-    CF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(sort_temp_.get(), temp, key_.get(), key_sorted_.get(),
-                                                  row_ids_.get(), order_.get(), static_cast<int>(list_rows_), 0, end_bit, st));
+           morton_bits_, frame_bits_, row_pos_.get(), row_label, row_both, key_.get(), row_ids_.get(), row_inv_.get());
+    CF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(sort_temp_.get(), sort_bytes_, key_.get(), key_sorted_.get(),
+                                                  row_ids_.get(), order_.get(), static_cast<int>(list_rows_), 0, end_bit(),
+                                                  st));
     launch(ctx, "stage_rows", dim3(static_cast<unsigned>((list_rows_ + 255) / 256)), dim3(256), 0, stage_list_kernel, rows,
-           list_rows_, general_bit, static_cast<const u64*>(key_sorted_.get()), order_.get(), row_pos_.get(), samples,
-           row_inv_.get(), ends_.get(), list_.get());
+           list_rows_, morton_bits_ + frame_bits_, static_cast<const u64*>(key_sorted_.get()), order_.get(), row_pos_.get(),
+           samples, row_inv_.get(), ends_.get(), list_.get());
 }
 
 void BinStager::run(cf_context* ctx, const DsView& ds, const Sample* samples, const LevelFeatures& lf, int c,

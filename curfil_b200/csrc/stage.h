@@ -28,18 +28,25 @@ class BinStager {
 public:
     // Whether the gather kernel serves such frames and thresholds.
     static bool gathers(const DsView& ds, int T);
-    // Orders the level's rows (row_base[n] + k is sample k of node n) and lays out the candidates of its
-    // n_chunks feature chunks of `chunk` features. With `both` the table has twice the rows: row rows + r is the
-    // flipped response of row r where row_both[r] (its sample has flip 2).
+    // Lays out a level of `rows` samples and n_chunks feature chunks of `chunk` features, and allocates everything that
+    // prepare() and run() use. With `both` the table has twice the rows: row rows + r is the flipped response of row r
+    // where row_both[r] (its sample has flip 2).
+    void reserve(cf_context* ctx, const DsView& ds, long long rows, bool both, const LevelFeatures& lf, int chunk,
+                 int n_chunks);
+    void release();
+    // Orders the level's rows (row_base[n] + k is sample k of node n) and lays out the candidates of its chunks.
     void prepare(cf_context* ctx, const DsView& ds, const Sample* samples, const NodeDesc* nodes_dev, int M,
-                 const long long* row_base_dev, long long rows, bool both, const LevelFeatures& lf, int chunk, int n_chunks,
-                 uint8_t* row_label, uint8_t* row_both);
+                 const long long* row_base_dev, const LevelFeatures& lf, uint8_t* row_label, uint8_t* row_both);
     // The bins of chunk c: feature f of the chunk and table row r at out[((f / 32) * table rows + r) * 32 + f % 32].
     void run(cf_context* ctx, const DsView& ds, const Sample* samples, const LevelFeatures& lf, int c, uint8_t* out);
 
 private:
+    // key bits that are sorted: kind 0 (gathered) or 1 (general) above the frame, with flipped rows also 3 (unused)
+    int end_bit() const { return morton_bits_ + frame_bits_ + (list_rows_ > sample_rows_ ? 2 : 1); }
     long long sample_rows_ = 0, list_rows_ = 0;
-    int chunk_ = 0, cap_ = 0;
+    int chunk_ = 0, n_chunks_ = 0, cap_ = 0;
+    int morton_bits_ = 0, frame_bits_ = 0;   // of a row's sort key
+    size_t sort_bytes_ = 0;
     bool padded_ = false;          // the level's thresholds and frames suit the gather kernel
     DevArray<unsigned long long> key_, key_sorted_;
     DevArray<int> row_pos_, row_ids_, order_;

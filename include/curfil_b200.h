@@ -131,7 +131,9 @@ typedef struct cf_eval_tuning {
                                     nodes) with T <= 63 and frames of up to 1.39 M pixels, a level is searched
                                     in two passes: the threshold bins of every (sample, feature) are computed
                                     in frame order into a byte table, then histogrammed node by node (huge
-                                    nodes in sample slices). 0: never; 2: always (T <= 255) */
+                                    nodes in sample slices). Where device memory is short the table
+                                    shrinks to narrower feature chunks, and at last the level is searched in
+                                    one pass. 0: never; 2: always (T <= 255) */
     int32_t stage_max_mb;        /* device memory of the staged bin table at most, 1..65536 MiB (default 8192; twice
                                     that where samples are evaluated both ways, flip 2); a level whose table is
                                     larger runs in feature chunks */
