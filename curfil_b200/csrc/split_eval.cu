@@ -116,6 +116,7 @@ struct EvalArgs {
     const uint8_t* row_label = nullptr;
     const uint8_t* row_both = nullptr;   // where samples have flip 2: row r's flipped bins are those of row
     long long both_rows = 0;             // both_rows + r if row_both[r]
+    bool flip_here = false;              // staged, and the flipped responses of samples with flip 2 are not
     // fused search over a copy of the samples sorted by (node, frame, Morton code): node n's samples
     // are rows row_base[n] .. of it; nullptr: the level's own array
     const Sample* sorted_samples = nullptr;
@@ -237,6 +238,28 @@ __device__ __noinline__ double score_from_cum_warp(const uint32_t* cum, int stri
     return normalize_score(__ddiv_rn(__dmul_rn(2.0, ig), __dadd_rn(hs, hc)));
 }
 
+// Counts the flipped responses of the samples of smps[0 .. N) with flip 2 into a tile's histogram of nf features x cp
+// classes x T + 1 bins. Out of line: only levels whose table has no room for the flipped rows call it.
+template <bool kAgg, int kPad>
+__device__ __noinline__ void count_flipped(const DsView ds, const Sample* smps, int N, const EvalFeat* params, const float* thr,
+                                           int row, int T, int nf, int cp, const uint8_t* class_id, uint32_t* bins) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int s0 = warp * 32; s0 < N; s0 += blockDim.x) {   // trip count uniform in a warp
+        const Sample smp = smps[min(s0 + lane, N - 1)];
+        const bool both = s0 + lane < N && smp.flip == 2;
+        if (!__any_sync(kFull, both)) continue;
+        const EvalPixel px = make_eval_pixel(ds, smp);
+        const int c = class_id[smp.label];
+        for (int f = 0; f < nf; f++) {
+            int key = -1;
+            if (both)
+                key = (f * cp + c) * (T + 1) +
+                      feature_bin(px, ds.width, ds.height, params[f], true, SortedBins<kPad>{thr + f * row, T});
+            bin_increment<kAgg>(bins, key);
+        }
+    }
+}
+
 constexpr int kExactList = 256;   // pairs of a tile listed for the exact score (more: scored where found)
 
 template <bool kAgg, int kPad, int kMinBlocks, bool kGrouped>
@@ -347,7 +370,7 @@ level_eval_kernel(EvalArgs a) {
         for (int f0 = item.f_begin; f0 < item.f_end; f0 += ft) {
             const int nf = min(ft, item.f_end - f0);
             // ---- stage the tile (the parameters and thresholds only where responses are computed)
-            const bool need_thr = !a.staged;
+            const bool need_thr = !a.staged || a.flip_here;
             for (int i = tid; i < nf && need_thr; i += blockDim.x) s_params[i] = make_eval_feat(a.packs[f0 + i]);
             const float* g_thr = a.sorted_thr + static_cast<long long>(f0) * T;
             if (!need_thr) {
@@ -425,6 +448,8 @@ level_eval_kernel(EvalArgs a) {
                             }
                     }
                 }
+                if (a.flip_here)
+                    count_flipped<kAgg, kPad>(a.ds, a.samples + sbase, N, s_params, s_thr, TPS, T, nf, cp, s_lid, s_bins);
             } else if constexpr (kGrouped) {
                 // ---- histogram, sample groups: the lanes of a warp take (sample, feature) pairs of a
                 // few consecutive samples (FL lanes per sample, FL = nf rounded up to a power of two,
@@ -1197,17 +1222,31 @@ void split_items_into_chunks(const std::vector<int>& node_counts, int chunk, int
     for (int c = n_chunks - 1; c >= 0; c--) chunk_begin[c] = std::min(chunk_begin[c], chunk_begin[c + 1]);
 }
 
-std::vector<StageTable> stage_tables(long long rows, int F, long long max_bytes) {
+std::vector<StageTable> stage_tables(long long rows, bool flips, int F, long long max_bytes) {
     const int tiles = (F + kStageTile - 1) / kStageTile;
-    std::vector<StageTable> out;
-    // chunks of whole tiles, as even as possible, then half as large
-    long long most = max_bytes / rows / kStageTile;
-    do {
+    constexpr int kWideTiles = kWideChunk / kStageTile;
+    // chunks of whole tiles, at most `most` of them, as even as possible
+    auto table = [&](long long most, bool both) {
         const int m = static_cast<int>(std::max<long long>(1, std::min<long long>(most, tiles)));
         const int n = (tiles + m - 1) / m, chunk = (tiles + n - 1) / n;
-        out.push_back(StageTable{chunk * kStageTile, (tiles + chunk - 1) / chunk});
-        most = chunk / 2;
-    } while (most >= 1);
+        return StageTable{chunk * kStageTile, (tiles + chunk - 1) / chunk, both};
+    };
+    std::vector<StageTable> out;
+    auto add = [&](StageTable t, int least) {   // t, then with chunks half as large, down to `least` tiles
+        for (int c = t.chunk / kStageTile; c >= least; c /= 2) {
+            t = table(c, t.both);
+            c = t.chunk / kStageTile;
+            out.push_back(t);
+        }
+    };
+    const StageTable one = table(max_bytes / rows / kStageTile, false);
+    if (flips) {
+        const long long most = max_bytes / (2 * rows) / kStageTile;
+        const StageTable both = table(most, true);
+        if (most >= std::min(kWideTiles, tiles) || (most >= 1 && both.n_chunks == one.n_chunks))
+            add(both, std::min(kWideTiles, both.chunk / kStageTile));
+    }
+    add(one, 1);
     return out;
 }
 
@@ -1260,25 +1299,27 @@ void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* s
     // stage_bins = 2 on every level. The bins are bytes (T <= 255)
     long long rows = 0;
     for (int c : node_counts) rows += c;
-    const long long table_rows = may_flip_both ? 2 * rows : rows, evals = table_rows * F;
+    const long long evals = (may_flip_both ? 2 * rows : rows) * F;
     const size_t frame_bytes = static_cast<size_t>(ds.n) * ds.plane * (3 * sizeof(float) + sizeof(int2));
-    bool stage = tuning.stage_bins != 0 && !sharded && T <= 255 && rows > 0 && table_rows < INT_MAX &&
+    bool stage = tuning.stage_bins != 0 && !sharded && T <= 255 && rows > 0 && rows < INT_MAX &&
                  (tuning.stage_bins == 2 || frame_bytes > ctx->l2_bytes ||
                   (BinStager::gathers(ds, T) && (evals >= kStageMinEvals ||
                                                  (evals >= kStageMinEvals / 4 && F >= 256 && M >= 64))));
-    StageTable table{0, 0};
+    StageTable table{0, 0, false};
     if (stage) {
         // everything pass 1 needs is allocated before its first launch: a table that does not fit the memory left
         // gives way to the next smaller one, and the last to the search in one pass, which needs none of this
         stage = false;
-        for (const StageTable& t : stage_tables(rows, F, static_cast<long long>(tuning.stage_max_mb) << 20)) {
+        for (const StageTable& t : stage_tables(rows, may_flip_both, F, static_cast<long long>(tuning.stage_max_mb) << 20)) {
+            const long long n = t.both ? 2 * rows : rows;
+            if (n >= INT_MAX) continue;
             try {
                 queue_.reserve(t.n_chunks);
                 row_base_.reserve(M + 1);
                 row_label_.reserve(rows);
-                if (may_flip_both) row_both_.reserve(rows);
-                stager_.reserve(ctx, ds, rows, may_flip_both, lf, t.chunk, t.n_chunks);
-                stage_.reserve(static_cast<size_t>(table_rows) * t.chunk);
+                if (t.both) row_both_.reserve(rows);
+                stager_.reserve(ctx, ds, rows, t.both, lf, t.chunk, t.n_chunks);
+                stage_.reserve(static_cast<size_t>(n) * t.chunk);
             } catch (const Error& e) {
                 if (e.code != CF_ERR_OOM) throw;
                 continue;
@@ -1388,10 +1429,11 @@ void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* s
            reinterpret_cast<NodeConsts*>(node_consts_.get()));
     if (stage) {
         args.staged = stage_.get();
-        args.staged_rows = table_rows;
+        args.staged_rows = table.both ? 2 * rows : rows;
         args.row_label = row_label_.get();
         args.row_base = row_base_.get();
-        args.row_both = may_flip_both ? row_both_.get() : nullptr;
+        args.row_both = table.both ? row_both_.get() : nullptr;
+        args.flip_here = may_flip_both && !table.both;
         args.both_rows = rows;
         for (int c = 0; c < n_chunks; c++) {
             if (c > 0) stager_.run(ctx, ds, samples, lf, c, stage_.get());

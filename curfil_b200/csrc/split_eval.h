@@ -88,13 +88,22 @@ constexpr double kStagedItemsPerSlot = 64.0;  // work items per resident CTA at 
 // one node 241 / 316, in 97 nodes 533 / 467, in 2000 nodes 1503 / 1088; 6 M (100 features) 460 / 481; 9.6 M in one
 // node 492 / 445; 30 M 877 / 773; 120 M in 97 nodes 3288 / 2208.
 constexpr long long kStageMinEvals = 1ll << 23;
-// The table of a staged level: n_chunks chunks of `chunk` features, one in memory at a time.
+// The table of a staged level: n_chunks chunks of `chunk` features, one in memory at a time. both: the flipped
+// responses of samples evaluated both ways (flip 2) have rows of their own, as many as there are samples; otherwise
+// pass 2 computes them.
 struct StageTable {
     int chunk, n_chunks;
+    bool both;
 };
 // The tables a level of `rows` samples may have, in the order in which they are tried until one can be allocated
-// (none: the level is searched in one pass).
-std::vector<StageTable> stage_tables(long long rows, int F, long long max_bytes);
+// (none: the level is searched in one pass). None holds more than max_bytes, or one tile of features if that is more.
+// Flipped rows are staged where they cost no further chunks or leave chunks of at least kWideChunk features. Staged is
+// the faster in either case (400 000 samples with flip 2, 1000 features, 500 nodes: 10.0 ms in one chunk, 11.2 in seven,
+// 20.8 with the flipped bins computed in four; 5200 x 331: 0.59 ms in four chunks, 0.95 computed in two), but a limit
+// below that keeps the number of chunks that the samples alone need, which callers and tests/test_gpu_staged.py reckon
+// with, and one too small for a tile of both leaves no other way.
+constexpr int kWideChunk = 4 * kStageTile;
+std::vector<StageTable> stage_tables(long long rows, bool flips, int F, long long max_bytes);
 // Splits every item at the chunk boundaries (multiples of `chunk` features) and orders the items
 // chunk by chunk, largest first within a chunk; chunk_begin[c] is the first order position of chunk c.
 void split_items_into_chunks(const std::vector<int>& node_counts, int chunk, int n_chunks,

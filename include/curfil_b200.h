@@ -134,9 +134,11 @@ typedef struct cf_eval_tuning {
                                     nodes in sample slices). Where device memory is short the table
                                     shrinks to narrower feature chunks, and at last the level is searched in
                                     one pass. 0: never; 2: always (T <= 255) */
-    int32_t stage_max_mb;        /* device memory of the staged bin table at most, 1..65536 MiB (default 8192; twice
-                                    that where samples are evaluated both ways, flip 2); a level whose table is
-                                    larger runs in feature chunks */
+    int32_t stage_max_mb;        /* device memory of the staged bin table at most, 1..65536 MiB (default 8192; never
+                                    less than 32 features of the level); a level whose table is larger runs
+                                    in feature chunks. Samples evaluated both ways (flip 2) have two rows
+                                    each where the limit leaves chunks of 128 features or costs no further
+                                    chunks; otherwise the second pass computes their flipped bins */
     int32_t sample_order;        /* levels searched in one pass: 1 (default) reads a copy of the samples sorted
                                     by (node, frame, Morton code of the pixel) where the integral images
                                     exceed the L2 cache, so a CTA's samples lie in a compact patch and

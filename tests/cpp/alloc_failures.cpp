@@ -2,7 +2,8 @@
 // allocations of this program's choice fail on the host. Prints one line per check and "<n> failures".
 //   1. each allocation of a call in turn fails once: the call gives the unlimited call's splits, or CF_ERR_OOM only
 //      where the search in one pass needs that allocation too, and the same call works again afterwards;
-//   2. allocations of a size and more fail: a smaller table, then the search in one pass.
+//   2. allocations of a size and more fail: a smaller table, then the search in one pass;
+//   3. stage_max_mb bounds the table whether or not samples are evaluated both ways, and the splits stay the same.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -14,11 +15,12 @@
 
 static bool armed = false;
 static int calls = 0, fail_at = -1;
-static size_t fail_from = ~size_t(0);
+static size_t fail_from = ~size_t(0), largest = 0;
 
 extern "C" cudaError_t __real_cudaMalloc(void** p, size_t bytes);
 extern "C" cudaError_t __wrap_cudaMalloc(void** p, size_t bytes) {
     if (armed && (calls++ == fail_at || bytes >= fail_from)) return cudaErrorMemoryAllocation;
+    if (armed && bytes > largest) largest = bytes;
     return __real_cudaMalloc(p, bytes);
 }
 
@@ -29,16 +31,17 @@ static void check(bool ok, const char* what, int flips, long long detail) {
 }
 
 struct Level {
-    static constexpr int kFrames = 3, kW = 96, kH = 72, kC = 11, kNodes = 5, kF = 64, kT = 20, kRows = 3000;
+    static constexpr int kFrames = 3, kW = 96, kH = 72, kC = 11, kNodes = 5, kT = 20, kRows = 3000;
     std::vector<uint8_t> rgb;
     std::vector<uint16_t> depth;
     std::vector<cf_sample> samples;
     std::vector<int64_t> offsets{0, 700, 701, 1500, 2900, kRows};
     std::vector<int8_t> features;
     std::vector<float> thresholds;
+    int F;
 
-    explicit Level(bool flips) : rgb(size_t(kFrames) * kW * kH * 3), depth(size_t(kFrames) * kW * kH), samples(kRows),
-                                 features(11 * kF), thresholds(kT * kF) {
+    explicit Level(bool flips, int kF = 64) : rgb(size_t(kFrames) * kW * kH * 3), depth(size_t(kFrames) * kW * kH), samples(kRows),
+                                 features(11 * kF), thresholds(kT * kF), F(kF) {
         std::mt19937 gen(7);
         auto pick = [&](int lo, int hi) { return std::uniform_int_distribution<int>(lo, hi)(gen); };
         for (auto& v : rgb) v = static_cast<uint8_t>(pick(0, 255));
@@ -85,7 +88,7 @@ struct Run {
         best.assign(Level::kNodes, cf_split{});
         cf_context_set_timing(ctx, 1);
         cf_context_reset_timing(ctx);
-        const cf_status s = cf_evaluate_best_splits(ds, Level::kNodes, level.offsets.data(), level.samples.data(), Level::kC, Level::kF,
+        const cf_status s = cf_evaluate_best_splits(ds, Level::kNodes, level.offsets.data(), level.samples.data(), Level::kC, level.F,
                                                     Level::kT, level.features.data(), level.thresholds.data(), best.data());
         double ms = 0;
         int64_t n = 0;
@@ -143,7 +146,7 @@ int main() {
         struct {
             size_t from;
             int64_t staged;
-        } limits[] = {{2 * tile + 1, 1}, {2 * tile, flips ? 0 : 2}, {tile, 0}};
+        } limits[] = {{2 * tile + 1, 1}, {2 * tile, 2}, {tile + 1, 2}, {tile, 0}};
         for (const auto& l : limits) {
             Run r(level, 2);
             armed = true;
@@ -156,6 +159,21 @@ int main() {
             check(same(best, want), "splits under a limit", flips, static_cast<long long>(l.from));
             std::printf("flips %d, allocations below %zu bytes: %lld launches of pass 1\n", flips, l.from, static_cast<long long>(staged));
             check((staged == 0) == (l.staged == 0), "passes under a limit", flips, static_cast<long long>(l.from));
+        }
+        // 20 tiles of 96 kB; the other allocations of the call are smaller
+        const Level wide(flips != 0, 640);
+        count_calls(wide, 0, want, &staged);
+        check(staged == 0, "one pass of the wide level", flips, staged);
+        for (int mb : {1, 2, 4}) {
+            Run r(wide, 2, mb);
+            armed = true;
+            largest = 0;
+            const cf_status s = r.call(best, &staged);
+            armed = false;
+            check(s == CF_OK && same(best, want), "splits with a bounded table", flips, mb);
+            check(staged >= 1 && largest <= size_t(mb) << 20, "bytes of a bounded table", flips, static_cast<long long>(largest));
+            std::printf("flips %d, stage_max_mb %d: %lld launches of pass 1, largest allocation %zu\n", flips, mb,
+                        static_cast<long long>(staged), largest);
         }
     }
     std::printf("%d failures\n", failures);
