@@ -74,6 +74,18 @@ METRIC = "train feature-evals/s"
 CPU_MODEL = None
 
 
+# The split search: level_eval (fused, or pass 2 reading staged bins), stage_bins (pass 1 of the staged levels) and
+# stage_general (pass 1 of the rows that its gather kernel does not serve).
+SEARCH_KERNELS = ("level_eval", "stage_bins", "stage_general")
+
+
+def split_search_times(kernel_time):
+    """(ms of the split search, {kernel: ms, launches, share}) from kernel_time(name) -> (ms, launches)."""
+    times = {k: kernel_time(k) for k in SEARCH_KERNELS}
+    total = sum(ms for ms, _ in times.values())
+    return total, {k: {"ms": ms, "launches": n, "share": ms / total if total else None} for k, (ms, n) in times.items()}
+
+
 def cpu_model():
     global CPU_MODEL
     if CPU_MODEL is None:
@@ -391,15 +403,12 @@ def headline(ctx, stream, local, rank, world, args, barrier, max_over_ranks, sum
     out["evals_per_step"] = total_evals / args.steps
     out["gpu_launches"] = int(launches)
     out["clocks"] = clocks.summary()
-    # the split search is level_eval (fused, or pass 2 reading staged bins) plus stage_bins (pass 1 of
-    # the staged levels); the roofline is that of the two together, with each kernel's share beside it
-    eval_ms, eval_launches = ctx.kernel_time("level_eval")
-    stage_ms, stage_launches = ctx.kernel_time("stage_bins")
-    out["kernel_ms"] = {k: ctx.kernel_time(k)[0] for k in ("level_eval", "stage_bins", "stage_rows", "node_consts",
-                                                            "gen_features", "sort_features", "route_flags",
-                                                            "route_scatter", "scan", "reduce_candidates")}
+    search_ms, search_kernels = split_search_times(ctx.kernel_time)
+    out["kernel_ms"] = {k: ctx.kernel_time(k)[0] for k in SEARCH_KERNELS + ("stage_plan", "stage_rows", "node_consts",
+                                                                            "gen_features", "sort_features",
+                                                                            "route_flags", "route_scatter", "scan",
+                                                                            "reduce_candidates")}
     bytes_per_eval = (BYTES_DEPTH_EVAL + BYTES_COLOR_EVAL) / 2.0
-    search_ms = eval_ms + stage_ms
     achieved = total_evals * bytes_per_eval / (search_ms / 1e3) / 1e9 if search_ms > 0 else None
     peak, peak_kind = load_peaks()
     traffic = None
@@ -408,14 +417,11 @@ def headline(ctx, stream, local, rank, world, args, barrier, max_over_ranks, sum
         for ln in open(tp):
             if ln.startswith("dram_bytes_per_feature_eval:"):
                 traffic = float(ln.split(":")[1]) * total_evals / max(1, args.steps)
-    out["roofline"] = {"bound": "hbm", "kernel": "split search (level_eval + stage_bins)", "achieved": achieved,
+    out["roofline"] = {"bound": "hbm", "kernel": "split search (level_eval + stage_bins + stage_general)", "achieved": achieved,
                        "peak": peak, "unit": "GB/s", "frac": (achieved / peak) if achieved else None,
                        "traffic": traffic, "traffic_per": "step (one level)", "peak_source": peak_kind,
                        "bytes_per_eval": bytes_per_eval, "ms_per_step": search_ms / max(1, args.steps),
-                       "kernels": {"level_eval": {"ms": eval_ms, "launches": eval_launches,
-                                                  "share": eval_ms / search_ms if search_ms else None},
-                                   "stage_bins": {"ms": stage_ms, "launches": stage_launches,
-                                                  "share": stage_ms / search_ms if search_ms else None}}}
+                       "kernels": search_kernels}
     out["levels"] = [{"level": s.level, "nodes": s.num_nodes, "samples": s.num_samples,
                       "ms": statistics.median(per_level[s.level]) if per_level[s.level] else None,
                       "feature_evals_per_s": s.num_samples * C3["features"] / (statistics.median(per_level[s.level]) / 1e3)
