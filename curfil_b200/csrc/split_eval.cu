@@ -1303,7 +1303,7 @@ void LevelEvaluator::evaluate(cf_context* ctx, const DsView& ds, const Sample* s
     const size_t frame_bytes = static_cast<size_t>(ds.n) * ds.plane * (3 * sizeof(float) + sizeof(int2));
     bool stage = tuning.stage_bins != 0 && !sharded && T <= 255 && rows > 0 && rows < INT_MAX &&
                  (tuning.stage_bins == 2 || frame_bytes > ctx->l2_bytes ||
-                  (BinStager::gathers(ds, T) && (evals >= kStageMinEvals ||
+                  (BinStager::gathers(ds, T) && (evals >= (F >= kStageMinFeatures ? 1 : 2) * kStageMinEvals ||
                                                  (evals >= kStageMinEvals / 4 && F >= 256 && M >= 64))));
     StageTable table{0, 0, false};
     if (stage) {

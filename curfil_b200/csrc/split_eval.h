@@ -83,10 +83,14 @@ void plan_level_items(const std::vector<int>& node_counts, int F, const EvalTuni
 constexpr int kStagedFeatures = 32;           // features per tile at most
 constexpr int kStagedBinsWords = 12288;       // histogram words per CTA
 constexpr double kStagedItemsPerSlot = 64.0;  // work items per resident CTA at most (16 and 256: the same)
-// Frames within L2: sample-feature pairs from which a level is staged; a quarter of that for levels of many nodes
-// and features, whose one-pass items are small. 24 frames 313x235, one pass against two, all in us: 2.4 M pairs in
-// one node 241 / 316, in 97 nodes 533 / 467, in 2000 nodes 1503 / 1088; 6 M (100 features) 460 / 481; 9.6 M in one
-// node 492 / 445; 30 M 877 / 773; 120 M in 97 nodes 3288 / 2208.
+// Frames within L2: sample-feature pairs from which a level is staged; twice that for fewer than kStageMinFeatures
+// features, which share a sample's part of the preparation among few; a quarter for levels of many nodes and features,
+// whose one-pass items are small. One pass against two, in us, on 24 frames 313x235: 2.4 M pairs in one node 241 / 316,
+// in 97 nodes 533 / 467, in 2000 nodes 1503 / 1088; 6 M (100 features) 460 / 481; 9.6 M in one node 492 / 445; 30 M 877 /
+// 773; 120 M in 97 nodes 3288 / 2208. Of 110 levels drawn over seven frame sets (1 to 40 frames, 160x120 to 1280x960)
+// those staged gain 3 to 83 %, except two of 100 features and 12 M pairs (699 / 750, 684 / 734; 18 M 808 / 764; 250
+// features and 12 M 651 / 616, 843 / 676).
+constexpr int kStageMinFeatures = 128;
 constexpr long long kStageMinEvals = 1ll << 23;
 // The table of a staged level: n_chunks chunks of `chunk` features, one in memory at a time. both: the flipped
 // responses of samples evaluated both ways (flip 2) have rows of their own, as many as there are samples; otherwise

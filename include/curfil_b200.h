@@ -127,13 +127,14 @@ typedef struct cf_eval_tuning {
                                     the same samples at once (their gathers share L2), but small items
                                     pay their setup more often */
     int32_t stage_bins;          /* 1 (default): when the integral images exceed the L2 cache, and on other levels
-                                    of at least 2^23 (sample, feature) pairs (2^21 with 256 features and 64
-                                    nodes) with T <= 63 and frames of up to 1.39 M pixels, a level is searched
-                                    in two passes: the threshold bins of every (sample, feature) are computed
-                                    in frame order into a byte table, then histogrammed node by node (huge
-                                    nodes in sample slices). Where device memory is short the table
-                                    shrinks to narrower feature chunks, and at last the level is searched in
-                                    one pass. 0: never; 2: always (T <= 255) */
+                                    of at least 2^23 (sample, feature) pairs (2^24 with fewer than 128
+                                    features, 2^21 with 256 features and 64 nodes) with T <= 63 and frames
+                                    of up to 1.39 M pixels, a level is searched in two passes: the threshold
+                                    bins of every (sample, feature) are computed in frame order into a byte
+                                    table, then histogrammed node by node (huge nodes in sample slices).
+                                    Where device memory is short the table shrinks to narrower feature
+                                    chunks, and at last the level is searched in one pass. 0: never;
+                                    2: always (T <= 255) */
     int32_t stage_max_mb;        /* device memory of the staged bin table at most, 1..65536 MiB (default 8192; never
                                     less than 32 features of the level); a level whose table is larger runs
                                     in feature chunks. Samples evaluated both ways (flip 2) have two rows

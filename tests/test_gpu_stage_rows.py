@@ -84,3 +84,32 @@ def test_general_bins_of_small_and_large_levels(ctx, T, rows):
     np.testing.assert_array_equal(out[2][1], out[0][1])
     for k in ("score", "feature", "threshold_index", "threshold"):
         np.testing.assert_array_equal(out[2][0][k], out[0][0][k], err_msg=k)
+
+
+@pytest.mark.parametrize("rows,F,T,staged", [(84000, 100, 20, False), (168000, 100, 20, True), (66000, 128, 20, True),
+                                             (65000, 128, 20, False), (66000, 128, 64, False)])
+def test_levels_within_l2_are_staged_by_their_size(ctx, rows, F, T, staged):
+    n, C, w, h = 3, 5, 97, 71
+    rgb, depth, labels = H.frames(seed=F, n=n, w=w, h=h, cells=9, classes=C)
+    ds = cf.Dataset.from_raw(ctx, rgb, depth)
+    rng = np.random.default_rng(rows + T)
+    offsets = np.array([0, rows // 3, rows], np.int64)
+    s = H.random_samples(rng, n, w, h, C, rows, depth=depth)
+    fe = H.random_features(rng, F)
+    r = cf.feature_responses(ds, s[:500], fe)
+    th = np.nan_to_num(r[np.arange(F), rng.integers(0, 500, (T, F))], nan=0.0).astype(np.float32)
+    out = {}
+    try:
+        for stage in (0, 1):
+            ctx.set_tuning(stage_bins=stage)
+            ctx.set_timing(True)
+            ctx.reset_timing()
+            out[stage] = cf.evaluate_best_splits(ds, offsets, s, C, fe, th)
+            assert (ctx.kernel_time("stage_bins")[1] > 0) == (staged and stage == 1)
+            ctx.set_timing(False)
+    finally:
+        ctx.set_timing(False)
+        ctx.set_tuning()
+        ds.close()
+    for k in ("score", "feature", "threshold_index", "threshold"):
+        np.testing.assert_array_equal(out[1][k], out[0][k], err_msg=k)
