@@ -113,3 +113,58 @@ def test_levels_within_l2_are_staged_by_their_size(ctx, rows, F, T, staged):
         ds.close()
     for k in ("score", "feature", "threshold_index", "threshold"):
         np.testing.assert_array_equal(out[1][k], out[0][k], err_msg=k)
+
+
+def assert_staged_equals_fused(ctx, ds, offsets, s, C, fe, th):
+    out = {}
+    try:
+        for stage in (0, 2):
+            ctx.set_tuning(stage_bins=stage)
+            ctx.set_timing(True)
+            ctx.reset_timing()
+            out[stage] = cf.level_left_counts(ds, offsets, s, C, fe, th)
+            assert (ctx.kernel_time("stage_bins")[1] > 0) == (stage == 2)
+            ctx.set_timing(False)
+    finally:
+        ctx.set_timing(False)
+        ctx.set_tuning()
+    np.testing.assert_array_equal(out[2][1], out[0][1])
+    for k in ("score", "feature", "threshold_index", "threshold"):
+        np.testing.assert_array_equal(out[2][0][k], out[0][0][k], err_msg=k)
+
+
+@pytest.mark.parametrize("T", [20, 32, 45, 64])
+def test_bins_on_padded_frames_equal_the_fused_search(ctx, T):
+    """Corners in the padding hold NaN colours and zero depth integrals: counts of boxes come out zero or negative."""
+    n, C, w, h, F = 4, 13, 70, 50, 160
+    rgb, depth, labels = H.frames(seed=T, n=n, w=w, h=h, cells=9, classes=C)
+    ds = cf.Dataset(ctx, n, 96, 72)
+    ds.upload_raw_padded(rgb, depth)
+    rng = np.random.default_rng(T)
+    offsets = np.array([0, 1, 900, 901, 3000], np.int64)
+    s = H.random_samples(rng, n, w, h, C, 3000, depth=depth, flips=True)
+    fe = H.random_features(rng, F)
+    r = cf.feature_responses(ds, s[:500], fe)
+    th = np.nan_to_num(r[np.arange(F), rng.integers(0, 500, (T, F))], nan=0.0).astype(np.float32)
+    assert_staged_equals_fused(ctx, ds, offsets, s, C, fe, th)
+    ds.close()
+
+
+@pytest.mark.parametrize("w,h", [(1399, 999), (1400, 1000)])
+def test_bins_on_large_frames_equal_the_fused_search(ctx, w, h):
+    """Frames on either side of the largest one whose byte offsets the gather kernel holds in floats."""
+    n, C, F, T = 1, 7, 96, 20
+    rng = np.random.default_rng(w)
+    rgb = rng.integers(0, 256, (n, h, w, 3), dtype=np.uint8)
+    depth = rng.integers(500, 5001, (n, h, w)).astype(np.uint16)
+    depth[rng.random(depth.shape) < 0.1] = 0
+    ds = cf.Dataset.from_raw(ctx, rgb, depth)
+    offsets = np.array([0, 700, 2500], np.int64)
+    s = H.random_samples(rng, n, w, h, C, 2500, depth=depth, flips=True)
+    s["x"][:200], s["y"][:200] = w - 1 - rng.integers(0, 60, 200), h - 1 - rng.integers(0, 60, 200)
+    s["depth"][:200] = np.float32(2.5)
+    fe = H.random_features(rng, F)
+    r = cf.feature_responses(ds, s[:500], fe)
+    th = np.nan_to_num(r[np.arange(F), rng.integers(0, 500, (T, F))], nan=0.0).astype(np.float32)
+    assert_staged_equals_fused(ctx, ds, offsets, s, C, fe, th)
+    ds.close()
