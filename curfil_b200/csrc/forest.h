@@ -51,7 +51,6 @@ struct cf_forest {
     cf::DevArray<int> d_tree_base;
     int leaf_stride = 0;             // floats of a leaf row: C rounded up to a multiple of 4, the rest 0
     cf::DevArray<float> leaves;      // [L][leaf_stride] normalised histograms (float, as convertTree stores them)
-    cf::DevArray<float> inv_mm;      // [65536] checked reciprocal of each depth in mm
     int64_t num_leaves = 0;
     // scratch of cf_predict_host
     cf::DevArray<uint8_t> raw_rgb;

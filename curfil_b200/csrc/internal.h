@@ -161,6 +161,10 @@ struct cf_context {
     // calls (the device's default pool gives everything back at each synchronisation)
     cudaMemPool_t scratch_pool = nullptr;
     static constexpr uint64_t kScratchKept = 256ull << 20;
+    // checked reciprocals of the depths in mm that predictions read (classify.cu), made with the first forest
+    cf::DevArray<float> inv_mm;
+    bool inv_mm_made = false;
+    std::mutex inv_mm_mu;
     std::mutex mu;
     struct KernelEvents {
         std::vector<std::pair<cudaEvent_t, cudaEvent_t>> pending;
