@@ -81,7 +81,7 @@ __device__ __forceinline__ u64 sign_pair(u64 v) { return (v & 0x8000000080000000
 // share in class order, and each normalises its own classes. The results are those of one thread per pixel.
 // With two threads per pixel half as many pixels are in flight per SM and their corners stay in L1 more often
 // (sector hit rate 47 -> 71 %), and 20 class sums instead of 40 fit in the registers beside the walk. The
-// kernel is bound by instruction issue (73 %) and the L1 tag pipe (73 %): 41 000 warp instructions for 32
+// kernel is bound by instruction issue (73 %) and L1 (77 % of its throughput): 41 000 warp instructions for 32
 // pixels of 10 trees, 65 700 before the walk used box_fast.cuh; 64 frames 640x480, 40 classes: 39.0 -> 28.4 ms.
 // kWide: a frame's byte offsets may pass 2^24, so corners are element indices in integers (wide_corners).
 template <int CMAX, int kPixels, int kSplit, bool kWide>

@@ -2,8 +2,9 @@
 //   - depth filling: RGBDImage::fillDepth runs four passes over the depth image, each replacing a
 //     missing (0) depth by its already-processed neighbour: from the right (x = W-2 .. 0 takes x+1),
 //     from the left (x = 1 .. W-1 takes x-1), from the top (y = 1 .. H-1 takes y-1), from the bottom
-//     (y = H-2 .. 0 takes y+1). Rows (and columns) are independent, so one thread runs one row (or
-//     column) of a pass; the result is bit-identical.
+//     (y = H-2 .. 0 takes y+1). Rows (and columns) are independent: a warp takes both passes of a row
+//     at once, a thread those of a column where rows without any depth leave something to fill; the
+//     result is bit-identical.
 //   - CIELab: the reference converts with Vigra's RGB2LabFunctor<double> (linear RGB in [0, 255]), a
 //     library not available here, so the published CIE 1976 L*a*b* definition is restated: RGB / 255
 //     -> XYZ with the ITU-R BT.709 primaries (D65), then L* = 116 f(Y/Yn) - 16, a* = 500 (f(X/Xn) -

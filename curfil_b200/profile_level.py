@@ -47,7 +47,8 @@ def main(argv=None):
     r = sn.run()
     torch.cuda.synchronize()
     torch.cuda.profiler.stop()
-    print("level ms", round(r["ms"], 3), {k: ctx.kernel_time(k) for k in ("stage_bins", "level_eval")}, flush=True)
+    print("level ms", round(r["ms"], 3),
+          {k: ctx.kernel_time(k) for k in ("stage_bins", "stage_general", "level_eval")}, flush=True)
 
 
 if __name__ == "__main__":
