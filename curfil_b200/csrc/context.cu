@@ -1,4 +1,5 @@
 // Context, error reporting and per-kernel CUDA-event timing.
+#include <algorithm>
 #include <cstring>
 
 #include "internal.h"
@@ -7,6 +8,30 @@ namespace cf {
 
 namespace {
 thread_local std::string g_last_error;
+
+// The live contexts' scratch pools; never destroyed, as contexts may go after the library's statics.
+struct Pools {
+    std::mutex mu;
+    std::vector<cudaMemPool_t> all;
+};
+Pools& scratch_pools() {
+    static Pools* pools = new Pools();
+    return *pools;
+}
+}  // namespace
+
+bool trim_scratch_pools() {
+    Pools& pools = scratch_pools();
+    std::lock_guard<std::mutex> lock(pools.mu);
+    bool any = false;
+    for (cudaMemPool_t pool : pools.all) {
+        uint64_t kept = 0, used = 0;
+        if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &kept) != cudaSuccess || kept == 0) continue;
+        if (!any) cudaDeviceSynchronize();   // blocks freed in stream order are unused once their stream has passed
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
+        any |= kept > used && cudaMemPoolTrimTo(pool, 0) == cudaSuccess;
+    }
+    return any;
 }
 
 void set_last_error(const std::string& msg) { g_last_error = msg; }
@@ -22,7 +47,12 @@ void destroy_context_now(cf_context* ctx) {
     for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
     if (ctx->spare_trainer && ctx->spare_trainer_free) ctx->spare_trainer_free(ctx->spare_trainer);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
-    if (ctx->scratch_pool) cudaMemPoolDestroy(ctx->scratch_pool);
+    if (ctx->scratch_pool) {
+        Pools& pools = scratch_pools();
+        std::lock_guard<std::mutex> lock(pools.mu);
+        pools.all.erase(std::find(pools.all.begin(), pools.all.end(), ctx->scratch_pool));
+        cudaMemPoolDestroy(ctx->scratch_pool);
+    }
     delete ctx;
 }
 
@@ -48,6 +78,11 @@ void* scratch_alloc(cf_context* ctx, size_t bytes, cudaStream_t stream) {
             if (e != cudaSuccess) {
                 cudaMemPoolDestroy(pool);
                 CF_CUDA_CHECK(e);
+            }
+            {
+                Pools& pools = scratch_pools();
+                std::lock_guard<std::mutex> pools_lock(pools.mu);
+                pools.all.push_back(pool);
             }
             ctx->scratch_pool = pool;
         }

@@ -56,6 +56,9 @@ cf_status guard(F&& f) {
     }
 }
 
+// Gives back the unused memory that the contexts' scratch pools keep; false if they keep none.
+bool trim_scratch_pools();
+
 // Owning device allocation (cudaMalloc); grows, never shrinks.
 class DeviceBuffer {
 public:
@@ -73,6 +76,10 @@ public:
         if (bytes == 0) return;
         void* p = nullptr;
         cudaError_t e = cudaMalloc(&p, bytes);
+        if (e == cudaErrorMemoryAllocation && trim_scratch_pools()) {
+            cudaGetLastError();
+            e = cudaMalloc(&p, bytes);
+        }
         if (e != cudaSuccess) {
             cudaGetLastError();
             fail(CF_ERR_OOM, "cudaMalloc(" + std::to_string(bytes) + ") failed: " + cudaGetErrorString(e));
@@ -158,7 +165,8 @@ struct cf_context {
     // of that workload (more CTAs on one node's samples at a time, sharing their gathers in L2).
     static cf_eval_tuning default_tuning() { return cf_eval_tuning{16, 7168, 0, 3, 4, 2048.0f, 1, 16384, 1, 8192, 1}; }
     // stream-ordered scratch of preprocessing; memory up to kScratchKept bytes stays with the pool between
-    // calls (the device's default pool gives everything back at each synchronisation)
+    // calls (the device's default pool gives everything back at each synchronisation), until an allocation of the
+    // library finds no memory
     cudaMemPool_t scratch_pool = nullptr;
     static constexpr uint64_t kScratchKept = 256ull << 20;
     // checked reciprocals of the depths in mm that predictions read (classify.cu), made with the first forest

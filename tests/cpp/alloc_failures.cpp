@@ -3,7 +3,8 @@
 //   1. each allocation of a call in turn fails once: the call gives the unlimited call's splits, or CF_ERR_OOM only
 //      where the search in one pass needs that allocation too, and the same call works again afterwards;
 //   2. allocations of a size and more fail: a smaller table, then the search in one pass;
-//   3. stage_max_mb bounds the table whether or not samples are evaluated both ways, and the splits stay the same.
+//   3. an allocation refused while a context keeps preprocessing scratch works again with that memory given back;
+//   4. stage_max_mb bounds the table whether or not samples are evaluated both ways, and the splits stay the same.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -159,6 +160,30 @@ int main() {
             check(same(best, want), "splits under a limit", flips, static_cast<long long>(l.from));
             std::printf("flips %d, allocations below %zu bytes: %lld launches of pass 1\n", flips, l.from, static_cast<long long>(staged));
             check((staged == 0) == (l.staged == 0), "passes under a limit", flips, static_cast<long long>(l.from));
+        }
+        {
+            Run r(level, 0);
+            const int w = 640, h = 480, frames = 4;   // L*a*b* scratch: 36 bytes a pixel, 44 MB
+            std::vector<uint8_t> rgb(size_t(frames) * w * h * 3, 90);
+            std::vector<uint16_t> depth(size_t(frames) * w * h, 1500);
+            cf_dataset* lab = nullptr;
+            check(cf_dataset_create(r.ctx, frames, w, h, &lab) == CF_OK &&
+                      cf_dataset_upload_raw_ex(lab, 0, frames, rgb.data(), depth.data(), 0, 1, 1) == CF_OK &&
+                      cf_context_synchronize(r.ctx) == CF_OK,
+                  "preprocessing", flips, 0);
+            size_t before = 0, after = 0, total = 0;
+            cudaMemGetInfo(&before, &total);
+            armed = true;
+            calls = 0;
+            fail_at = 0;
+            const cf_status s = r.call(best);
+            armed = false;
+            fail_at = -1;
+            cudaMemGetInfo(&after, &total);
+            check(s == CF_OK && same(best, want), "a refused allocation with scratch kept", flips, s);
+            check(after > before + (size_t(16) << 20), "scratch given back", flips, static_cast<long long>(after) - static_cast<long long>(before));
+            check(cf_dataset_upload_raw_ex(lab, 0, frames, rgb.data(), depth.data(), 0, 1, 1) == CF_OK, "preprocessing again", flips, 0);
+            cf_dataset_destroy(lab);
         }
         // 20 tiles of 96 kB; the other allocations of the call are smaller
         const Level wide(flips != 0, 640);
